@@ -18,6 +18,7 @@ struct MatchArgs {
     int nbx_al;            // blocks whose x = bs*kx needs no clamp
     int tile_pitch;        // shared tile row pitch in floats (tiled kernel)
     int chunks;            // ceil((2*range+1)/4)
+    int tiles_x;           // scan kernel: tiles per row; one more column of CTAs takes the clamped blocks
     int2 *list;            // [nby*nbx][8]: (x, y | z << 24)
     float *errs;           // [nby*nbx][8]: distances of the spatial list (radius > 0)
     int self_incl;         // 1: insert the block itself here (radius 0)
@@ -58,7 +59,8 @@ struct FilterArgs {
 struct BatchEntry {
     MatchArgs m;                      // tile_pitch, chunks and self_incl set; bs 4 or 8
     FilterArgs f;
-    int tiles_x;                      // match tiles per tile row (31 or 16 block columns each)
+    int tiles_x;                      // match items per tile row: m.tiles_x tiles, and one for the
+                                      // clamped last block column where there is one
     int match_items;                  // match tiles (kBatchMatchRows block rows each)
     int filter_items;                 // filter chunks (kBatchGroups groups each)
     long long first_match, first_filter;  // first item number of each kind
@@ -74,6 +76,9 @@ struct BatchArgs {
     unsigned wait_polls;              // polls (about 0.1 us apart) before a wait gives up
     int unsatisfiable;                // testing: entry 0's chunks wait for one tile more than it has
 };
+
+// Largest dynamic shared memory of a CTA on sm_100 (227 KB), less 1 KB for static variables.
+constexpr unsigned kSmemOptIn = 226 * 1024;
 
 constexpr int kBatchGroups = 128;     // groups per filter chunk
 constexpr int kBatchMatchRows = 8;    // block rows (warps) per match tile

@@ -40,12 +40,12 @@ cudaError_t launch_tc_fallback(MatchArgs a, cudaStream_t st);
 int tc_debug_cols(const MatchArgs &a);
 int pilot_device(const zb3d_pilot *p);
 size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
-size_t match_tile2_bytes_rows(const MatchArgs &a, int rows_per_cta);
+bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta);
+bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta);
 size_t batch_match_smem(const MatchArgs &m);
 size_t batch_filter_smem(bool final_);
 cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, size_t filter_smem,
                          cudaStream_t st);
-cudaError_t launch_clamped_column(MatchArgs a, cudaStream_t st);
 cudaError_t filter_precision_init(int dev);
 size_t filter_precision_stack_floats(long long nblocks);
 cudaError_t launch_filter_precision(const FilterArgs &a, bool final_, float *stack, float *basic, float *weight,
@@ -437,7 +437,7 @@ cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src) {
 // fastest launch configuration of the matching stage for a plane geometry,
 // timed on this GPU.  Every candidate gives bit-identical lists, so the choice
 // never changes results.  Cache file: $ZB3D_TUNE_CACHE, else
-// $XDG_CACHE_HOME/zb3d/tune-v2.txt or ~/.cache/zb3d/tune-v2.txt; one line per key
+// $XDG_CACHE_HOME/zb3d/tune-v3.txt or ~/.cache/zb3d/tune-v3.txt; one line per key
 // "key form rows".  ZB3D_AUTOTUNE=0 turns the timing off (defaults are used).
 struct TuneCache {
     std::mutex mu;
@@ -455,9 +455,9 @@ std::string tune_path() {
     const char *p = getenv("ZB3D_TUNE_CACHE");
     if (p && *p) return p;
     const char *x = getenv("XDG_CACHE_HOME");
-    if (x && *x) return std::string(x) + "/zb3d/tune-v2.txt";
+    if (x && *x) return std::string(x) + "/zb3d/tune-v3.txt";
     const char *h = getenv("HOME");
-    if (h && *h) return std::string(h) + "/.cache/zb3d/tune-v2.txt";
+    if (h && *h) return std::string(h) + "/.cache/zb3d/tune-v3.txt";
     return "";
 }
 
@@ -488,22 +488,37 @@ void tune_store(TuneCache &c, const std::string &key, int form, int rows) {
     fclose(fp);
 }
 
-// Whether the packed SSD kernel's tile for `rows` block rows per CTA fits (that kernel
-// takes up to 8 warps; the other tiled kernels take at most 4).
-bool tiled2_rows_fit(const Entry &e, int rows) {
-    if (e.metric != M_SSD || (e.bs != 4 && e.bs != 8)) return false;
+// Whether the scan kernel takes the entry with `rows` block rows per CTA.
+bool entry_scan_fits(const Entry &e, int rows) {
     MatchArgs t{};
     t.bs = e.bs;
     t.range = e.range;
     t.chunks = (2 * e.range + 1 + 3) / 4;
     t.tile_pitch = 128 + 4 * t.chunks;
-    return match_tile2_bytes_rows(t, rows) <= 200 * 1024;
+    return scan_rows_fit(t, e.metric, rows);
+}
+
+// Whether two CTAs of that shape fit an SM's shared memory.
+bool entry_scan_fits2(const Entry &e, int rows) {
+    MatchArgs t{};
+    t.bs = e.bs;
+    t.range = e.range;
+    t.chunks = (2 * e.range + 1 + 3) / 4;
+    t.tile_pitch = 128 + 4 * t.chunks;
+    return scan_rows_fit2(t, e.metric, rows);
+}
+
+// CTAs of the scan kernel for the entry.
+long long scan_ctas(const Entry &e, int rows) {
+    const int nbw = e.bs == 4 ? 31 : 16;
+    return (long long)((e.nbx_al + nbw - 1) / nbw) * ((e.nby + rows - 1) / rows);
 }
 
 // Chooses e.form / e.rows: FP32 scan with 2 or 4 block rows per CTA (tiled block
-// steps 4 and 8), also 8 for the packed SSD kernel, or the tensor-core form (ssd,
-// where eligible), by timing
-// each on a synthetic plane of the entry's geometry with slot s's buffers.
+// steps 4 and 8) or, for the scan kernel (ssd, sad), 8 block rows or fewer (its CTAs always
+// have 8 warps; fewer rows split each block's candidate rows, which helps a plane whose CTAs
+// do not fill the GPU), or the tensor-core form (ssd, where eligible), by timing each on a
+// synthetic plane of the entry's geometry with slot s's buffers.
 void tune_entry(Filter *f, Slot &s, Entry &e) {
     e.rows = 4;
     MatchArgs ga{};
@@ -515,10 +530,21 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     const bool tiled = e.bs == 4 || e.bs == 8;
     e.form = (f->match_form == 1 && tc_ok) ? 1 : 0;
     std::vector<std::pair<int, int>> cands;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device);
     if (f->match_form != 1 || !tc_ok) {
-        if (tiled)
+        if (tiled && !entry_scan_fits(e, 1))
             for (int r : {2, 4}) cands.push_back({0, r});
-        if (tiled2_rows_fit(e, 8)) cands.push_back({0, 8});
+        // from 8 rows down; a plane that already has 4 waves of CTAs (2 per SM) gains nothing
+        // from more of them, and a tile that leaves one CTA per SM is only taken for want of others
+        int last = 0;
+        for (int r = 8; r >= 1; r >>= 1) {
+            if (!entry_scan_fits(e, r)) continue;
+            if (last && !entry_scan_fits2(e, last)) cands.clear();
+            else if (last && scan_ctas(e, last) >= 8LL * sms) break;
+            cands.push_back({0, r});
+            last = r;
+        }
     }
     if (tc_ok && f->match_form != 0) cands.push_back({1, 4});
     if (cands.size() < 2) return;
@@ -542,7 +568,10 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     auto it = c.best.find(key);
     if (it != c.best.end()) {
         const int form = it->second.first, rows = it->second.second;
-        if ((form == 0 && (rows == 2 || rows == 4 || (rows == 8 && tiled2_rows_fit(e, 8)))) || (form == 1 && tc_ok)) {
+        const bool scan = entry_scan_fits(e, 1);
+        if ((form == 0 && !scan && (rows == 2 || rows == 4)) ||
+            (form == 0 && scan && (rows == 1 || rows == 2 || rows == 4 || rows == 8) && entry_scan_fits(e, rows)) ||
+            (form == 1 && tc_ok)) {
             e.form = form;
             e.rows = rows;
         }
@@ -565,6 +594,7 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
                         cudaMemcpyHostToDevice) == cudaSuccess;
     float best_ms = 3.0e38f;
     int bform = -1, brows = e.rows;
+    std::vector<std::pair<float, std::pair<int, int>>> times;
     for (const auto &cand : cands) {
         if (!ok) break;
         Entry t = e;
@@ -583,12 +613,18 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
             cudaGetLastError();
             continue;
         }
-        if (lo < best_ms) {
-            best_ms = lo;
-            bform = cand.first;
-            brows = cand.second;
-        }
+        if (lo < best_ms) best_ms = lo;
+        times.push_back({lo, cand});
     }
+    // the first candidate within 20% of the fastest: fewer block rows per CTA make one plane's
+    // launch shorter by filling the GPU, but cost more in all (every range of candidate rows
+    // builds a list of its own), which shows as soon as other streams fill it (640x480 at
+    // block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3 streams)
+    for (const auto &t : times)
+        if (bform < 0 && t.first <= 1.2f * best_ms) {
+            bform = t.second.first;
+            brows = t.second.second;
+        }
     ok = ok && bform >= 0;
     if (a) cudaEventDestroy(a);
     if (b) cudaEventDestroy(b);
@@ -931,7 +967,7 @@ bool batch_eligible(const Filter *f, const Entry &en) {
     m.range = en.range;
     m.chunks = (2 * en.range + 1 + 3) / 4;
     m.tile_pitch = 128 + 4 * m.chunks;
-    return match_tile2_bytes_rows(m, kBatchMatchRows) <= 200 * 1024;
+    return scan_rows_fit(m, M_SSD, kBatchMatchRows);
 }
 
 
@@ -1126,15 +1162,13 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
             fa.acc_frame_stride = (long long)en.plane_elems;
             fa.acc_plane_stride = (long long)en.plane_elems;
             const int nbw = en.bs == 4 ? 31 : 16;
-            B.tiles_x = (en.nbx_al + nbw - 1) / nbw;
+            m.tiles_x = (en.nbx_al + nbw - 1) / nbw;
+            B.tiles_x = m.tiles_x + (en.nbx_al != en.nbx ? 1 : 0);
             B.match_items = B.tiles_x * ((en.nby + kBatchMatchRows - 1) / kBatchMatchRows);
             B.filter_items = (int)((en.nblocks + kBatchGroups - 1) / kBatchGroups);
             B.first_match = nm;
             nm += B.match_items;
             smem[g] = std::max(smem[g], batch_match_smem(m));
-            // the clamped last column, before the batch launch (the batch's lists are complete
-            // when its filter chunks read them)
-            if (en.nbx_al != en.nbx && (ce = launch_clamped_column(m, st)) != cudaSuccess) break;
             ++idx;
         }
         long long nf = nm;

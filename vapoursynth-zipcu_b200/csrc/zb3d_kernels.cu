@@ -381,7 +381,7 @@ __device__ __forceinline__ int batch_entry_of(const BatchArgs &b, long long item
 // PHASE 1: the match tiles (kBatchMatchRows warps per CTA); PHASE 2: the filter chunks
 // (4 warps per CTA).  Each phase is one persistent launch with its own register budget.
 template <bool FINAL, int T2D, int T1D, int PHASE>
-__global__ void __launch_bounds__(PHASE == 1 ? kBatchMatchRows * 32 : 128) zb_batch(BatchArgs b) {
+__global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : 128) zb_batch(BatchArgs b) {
     extern __shared__ __align__(16) float dyn[];  // matching tile, or the Wiener coefficient buffer
     __shared__ float tbuf[PHASE == 1 ? 1 : kFilterWarps * 2 * kGroupBuf];
     __shared__ long long s_item;
@@ -400,10 +400,14 @@ __global__ void __launch_bounds__(PHASE == 1 ? kBatchMatchRows * 32 : 128) zb_ba
             const BatchEntry &E = b.entries[e];
             const int local = (int)(item - E.first_match);
             const int bx = local % E.tiles_x, by = local / E.tiles_x;
-            if (E.m.bs == 4)
-                match_tiled2_tile<true, 4>(E.m, bx, by, dyn);
-            else
-                match_tiled2_tile<false, 8>(E.m, bx, by, dyn);
+            if (bx == E.m.tiles_x) {  // the clamped last block column
+                const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
+                if (cy < E.m.nby) column_block<M_SSD>(E.m, cy);
+            } else if (E.m.bs == 4) {
+                scan_tile<M_SSD, true, 4>(E.m, bx, by, kBatchMatchRows, dyn);
+            } else {
+                scan_tile<M_SSD, false, 8>(E.m, bx, by, kBatchMatchRows, dyn);
+            }
             __threadfence();  // each thread's list stores before the tile's count
             __syncthreads();
             if (threadIdx.x == 0) atomicAdd(&b.match_done[e], 1u);
@@ -501,12 +505,16 @@ cudaError_t launch_finish(const unsigned long long *num, const unsigned long lon
 
 // Bytes of dynamic shared memory a batch entry needs: its matching tile (kBatchMatchRows
 // block rows), and the Wiener coefficient buffer of its filter chunks.
-size_t batch_match_smem(const MatchArgs &m) { return match_tile2_bytes(m, kBatchMatchRows); }
+size_t batch_match_smem(const MatchArgs &m) { return scan_smem_bytes(m, kBatchMatchRows); }
 size_t batch_filter_smem(bool final_) { return final_ ? (size_t)(128 / 16) * kCoeffBuf * sizeof(float) : 0; }
 
 template <class K>
 static cudaError_t launch_batch_k(K k, const BatchArgs &b, int threads, size_t smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same limit at every launch (see launch_scan_t), less the static buffers
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, k);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemOptIn - fa.sharedSizeBytes));
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 148, per = 1;
     cudaGetDevice(&dev);
@@ -525,7 +533,7 @@ cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t matc
                          cudaStream_t st) {
     if (t2d != T_DCT || t1d != T_DCT) return cudaErrorNotSupported;
     cudaError_t e = launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 1> : zb_batch<false, T_DCT, T_DCT, 1>, b,
-                                   kBatchMatchRows * 32, match_smem, st);
+                                   kScanWarps * 32, match_smem, st);
     if (e != cudaSuccess) return e;
     b.next += 1;
     return launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 2> : zb_batch<false, T_DCT, T_DCT, 2>, b, 128,

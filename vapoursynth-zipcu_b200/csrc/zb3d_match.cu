@@ -125,11 +125,26 @@ __global__ void __launch_bounds__(128) zb_match_tiled(MatchArgs a) {
     store_list(a, (long long)by * a.nbx + kx, xb, y, e, q);
 }
 
-// Up to 8 block rows (warps) per CTA; 2 CTAs of 8 warps fit the register file.
-template <bool SHARED, int BS>
-__global__ void __launch_bounds__(256, 2) zb_match_tiled2(MatchArgs a) {
+// The column on its own, beside the tiled kernels of the metrics that zb_match_scan does not take.
+template <int M>
+__global__ void __launch_bounds__(128) zb_match_column(MatchArgs a) {
+    const int by = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (by < a.nby) column_block<M>(a, by);  // whole warps
+}
+
+// Spatial SSD / SAD matching at block_step 4 and 8 (scan_tile), `rows` block rows per CTA of 8
+// warps.  Where the plane's width leaves a clamped last block column, one more column of CTAs
+// scans it, a warp per block, instead of a launch of its own (11 to 17 us, most of it the
+// latency of one warp per block).
+template <int M, bool SHARED, int BS>
+__global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a, int rows) {
     extern __shared__ __align__(16) float tile[];
-    match_tiled2_tile<SHARED, BS>(a, blockIdx.x, blockIdx.y, tile);
+    if ((int)blockIdx.x == a.tiles_x) {
+        const int warp = threadIdx.x >> 5, by = blockIdx.y * rows + warp;
+        if (warp < rows && by < a.nby) column_block<M>(a, by);
+        return;
+    }
+    scan_tile<M, SHARED, BS>(a, blockIdx.x, blockIdx.y, rows, tile);
 }
 
 // Spatial matching for block steps the tiled kernels do not take (and the blocks the
@@ -178,89 +193,6 @@ __global__ void __launch_bounds__(128) zb_match_global(MatchArgs a) {
                        e, q);
     }
     if (hh) return;
-    const long long bi = (long long)by * a.nbx + kx;
-    const int self = pack_pos(x, y);
-    if (a.self_incl) {
-        bool found = false;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) found |= (q[i] == self);
-        if (!found) {
-#pragma unroll
-            for (int i = 7; i > 0; --i) {
-                e[i] = e[i - 1];
-                q[i] = q[i - 1];
-            }
-            e[0] = 0.0f;
-            q[0] = self;
-        }
-    }
-    const int zr = a.radius << 24;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) a.list[bi * 8 + i] = make_int2(pos_x(q[i]), pos_y(q[i]) | zr);
-    if (a.errs) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a.errs[bi * 8 + i] = e[i];
-    }
-}
-
-// The clamped last block column (x = W - 8) that the tiled kernels leave out: one warp per
-// block.  Its candidate rows are split into 16 consecutive ranges in order, one per lane
-// pair, each scanned in the reference's order into a list of its own; the lists are then
-// merged in row order, a later range's entries inserted (strict less) after the earlier
-// ranges', which is the list of one scan over all the rows.
-template <int M>
-__global__ void __launch_bounds__(128) zb_match_column(MatchArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int by = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (by >= a.nby) return;  // whole warps
-    const int hh = lane & 1, pr = lane >> 1;
-    const int W = a.w, H = a.h, R = a.range;
-    const int kx = a.nbx - 1;
-    const int x = min(a.bs * kx, W - 8), y = min(a.bs * by, H - 8);
-    const unsigned pm = 3u << (lane & 30);
-    const float *plane = a.frames + (long long)a.radius * a.fstride + 4 * hh;
-
-    float c[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) c[i][j] = __ldg(plane + (long long)(y + i) * a.pitch + x + j);
-    const float st = ref_stat<M>(c, pm);
-    float e[8];
-    int q[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        e[i] = ZB_FLT_MAX;
-        q[i] = 0;
-    }
-    const int top = max(y - R, 0), bottom = min(y + R, H - 8);
-    const int per = (bottom - top + 16) / 16;
-    const int r0 = top + pr * per, r1 = min(r0 + per - 1, bottom);
-    if (r0 <= r1) {
-        if constexpr (M == M_SSD) {
-            float2 nc[4][4];
-            neg_pairs(c, nc);
-            scan_window_ssd2(plane, a.pitch, max(x - R, 0), min(x + R, W - 8), r0, r1, nc, pm, e, q);
-        } else {
-            scan_window<M>(plane, a.pitch, max(x - R, 0), min(x + R, W - 8), r0, r1, c, st, pm, e, q);
-        }
-    }
-#pragma unroll
-    for (int k = 1; k < 16; k <<= 1) {
-        float oe[8];
-        int oq[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            oe[i] = __shfl_down_sync(kFull, e[i], 2 * k);
-            oq[i] = __shfl_down_sync(kFull, q[i], 2 * k);
-        }
-        if ((pr & (2 * k - 1)) == 0) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (oe[i] < e[7]) top8_insert(e, q, oe[i], oq[i]);
-        }
-    }
-    if (lane != 0) return;
     const long long bi = (long long)by * a.nbx + kx;
     const int self = pack_pos(x, y);
     if (a.self_incl) {
@@ -397,33 +329,53 @@ static cudaError_t launch_tiled_t(const MatchArgs &a, int rows_per_cta, cudaStre
     const int gy = (a.nby + rows_per_cta - 1) / rows_per_cta;
     const size_t smem = match_tile_bytes(a, rows_per_cta);
     auto k = zb_match_tiled<M, SHARED, BS>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptIn);
     if (e != cudaSuccess) return e;
     k<<<dim3(gx, gy), rows_per_cta * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <bool SHARED, int BS>
-static cudaError_t launch_tiled2_t(const MatchArgs &a, int rows_per_cta, cudaStream_t st) {
-    constexpr int NBW = SHARED ? 31 : 16;
-    const int gx = (a.nbx_al + NBW - 1) / NBW;
-    const int gy = (a.nby + rows_per_cta - 1) / rows_per_cta;
-    const size_t smem = match_tile2_bytes(a, rows_per_cta);
-    auto k = zb_match_tiled2<SHARED, BS>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Whether the scan kernel takes an entry with this many block rows per CTA: ssd and sad at
+// block_step 4 and 8, a tile that fits shared memory.
+bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta) {
+    if ((metric != M_SSD && metric != M_SAD) || (a.bs != 4 && a.bs != 8)) return false;
+    return scan_smem_bytes(a, rows_per_cta) <= kSmemOptIn;
+}
+
+// Whether two such CTAs share an SM (227 KB, 1 KB of it reserved per CTA).
+bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta) {
+    return scan_rows_fit(a, metric, rows_per_cta) && scan_smem_bytes(a, rows_per_cta) <= kSmemOptIn / 2;
+}
+
+template <int M, bool SHARED, int BS>
+static cudaError_t launch_scan_t(const MatchArgs &a, int rows, cudaStream_t st) {
+    auto k = zb_match_scan<M, SHARED, BS>;
+    // the same limit at every launch: a limit of this launch's size would race with other
+    // threads' launches of the same kernel
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptIn);
     if (e != cudaSuccess) return e;
-    k<<<dim3(gx, gy), rows_per_cta * 32, smem, st>>>(a);
+    const int gx = a.tiles_x + (a.nbx_al != a.nbx ? 1 : 0), gy = (a.nby + rows - 1) / rows;
+    k<<<dim3(gx, gy), kScanWarps * 32, scan_smem_bytes(a, rows), st>>>(a, rows);
     return cudaGetLastError();
+}
+
+// Block rows per CTA of the scan: the asked power of two, or fewer where its tile does not
+// fit; 0 where none does.
+static int scan_rows(const MatchArgs &a, int metric, int rows) {
+    int r = rows >= 8 ? 8 : rows >= 4 ? 4 : rows >= 2 ? 2 : 1;
+    while (r > 0 && !scan_rows_fit(a, metric, r)) r >>= 1;
+    return r;
 }
 
 template <int M>
-static cudaError_t launch_tiled_m(const MatchArgs &a, int rows_per_cta, cudaStream_t st) {
-    if constexpr (M == M_SSD) {
-        // SSD at block_step 4 / 8: the packed FP32x2 kernel whenever its two tiles fit
-        if (match_tile2_bytes(a, rows_per_cta) <= 200 * 1024)
-            return a.bs == 8 ? launch_tiled2_t<false, 8>(a, rows_per_cta, st)
-                             : launch_tiled2_t<true, 4>(a, rows_per_cta, st);
+static cudaError_t launch_tiled_m(MatchArgs a, int rows_per_cta, cudaStream_t st) {
+    if constexpr (M == M_SSD || M == M_SAD) {
+        if (const int rows = scan_rows(a, M, rows_per_cta)) {
+            a.tiles_x = scan_tiles_x(a);
+            return a.bs == 8 ? launch_scan_t<M, false, 8>(a, rows, st) : launch_scan_t<M, true, 4>(a, rows, st);
+        }
     }
+    rows_per_cta = std::min(rows_per_cta, 4);
     if (a.bs == 8) return launch_tiled_t<M, false, 8>(a, rows_per_cta, st);
     if constexpr (Shareable<M>::value) return launch_tiled_t<M, true, 4>(a, rows_per_cta, st);
     return launch_tiled_t<M, false, 4>(a, rows_per_cta, st);
@@ -490,7 +442,7 @@ cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_til
         default: e = launch_tiled_m<M_SSD_NORM>(a, rows_per_cta, st); break;
         }
         if (e != cudaSuccess) return e;
-        if (a.nbx_al == a.nbx) goto temporal;
+        if (a.nbx_al == a.nbx || scan_rows(a, metric, rows_per_cta)) goto temporal;
         switch (metric) {  // the clamped last column
         case M_SSD: e = launch_column_m<M_SSD>(a, st); break;
         case M_SAD: e = launch_column_m<M_SAD>(a, st); break;
@@ -522,13 +474,5 @@ temporal:
     }
     return e;
 }
-
-// The clamped last block column of an entry (x = w - 8), which the tiled kernels leave out.
-cudaError_t launch_clamped_column(MatchArgs a, cudaStream_t st) {
-    a.self_incl = a.radius == 0;
-    return launch_column_m<M_SSD>(a, st);
-}
-
-size_t match_tile2_bytes_rows(const MatchArgs &a, int rows_per_cta) { return match_tile2_bytes(a, rows_per_cta); }
 
 }  // namespace zb

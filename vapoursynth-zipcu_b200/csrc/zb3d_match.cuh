@@ -358,4 +358,85 @@ __device__ __forceinline__ void neg_pairs(const float (&c)[8][4], float2 (&nc)[4
         for (int j = 0; j < 4; ++j) nc[k][j] = make_float2(-c[2 * k][j], -c[2 * k + 1][j]);
 }
 
+// The clamped last block column (x = W - 8) that the tiled kernels leave out: one warp per
+// block.  Its candidate rows are split into 16 consecutive ranges in order, one per lane
+// pair, each scanned in the reference's order into a list of its own; the lists are then
+// merged in row order, a later range's entries inserted (strict less) after the earlier
+// ranges', which is the list of one scan over all the rows.
+template <int M>
+__device__ __forceinline__ void column_block(const MatchArgs &a, int by) {
+    const int lane = threadIdx.x & 31;
+    const int hh = lane & 1, pr = lane >> 1;
+    const int W = a.w, H = a.h, R = a.range;
+    const int kx = a.nbx - 1;
+    const int x = min(a.bs * kx, W - 8), y = min(a.bs * by, H - 8);
+    const unsigned pm = 3u << (lane & 30);
+    const float *plane = a.frames + (long long)a.radius * a.fstride + 4 * hh;
+
+    float c[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[i][j] = __ldg(plane + (long long)(y + i) * a.pitch + x + j);
+    const float st = ref_stat<M>(c, pm);
+    float e[8];
+    int q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        e[i] = ZB_FLT_MAX;
+        q[i] = 0;
+    }
+    const int top = max(y - R, 0), bottom = min(y + R, H - 8);
+    const int per = (bottom - top + 16) / 16;
+    const int r0 = top + pr * per, r1 = min(r0 + per - 1, bottom);
+    if (r0 <= r1) {
+        if constexpr (M == M_SSD) {
+            float2 nc[4][4];
+            neg_pairs(c, nc);
+            scan_window_ssd2(plane, a.pitch, max(x - R, 0), min(x + R, W - 8), r0, r1, nc, pm, e, q);
+        } else {
+            scan_window<M>(plane, a.pitch, max(x - R, 0), min(x + R, W - 8), r0, r1, c, st, pm, e, q);
+        }
+    }
+#pragma unroll
+    for (int k = 1; k < 16; k <<= 1) {
+        float oe[8];
+        int oq[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            oe[i] = __shfl_down_sync(kFull, e[i], 2 * k);
+            oq[i] = __shfl_down_sync(kFull, q[i], 2 * k);
+        }
+        if ((pr & (2 * k - 1)) == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (oe[i] < e[7]) top8_insert(e, q, oe[i], oq[i]);
+        }
+    }
+    if (lane != 0) return;
+    const long long bi = (long long)by * a.nbx + kx;
+    const int self = pack_pos(x, y);
+    if (a.self_incl) {
+        bool found = false;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) found |= (q[i] == self);
+        if (!found) {
+#pragma unroll
+            for (int i = 7; i > 0; --i) {
+                e[i] = e[i - 1];
+                q[i] = q[i - 1];
+            }
+            e[0] = 0.0f;
+            q[0] = self;
+        }
+    }
+    const int zr = a.radius << 24;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a.list[bi * 8 + i] = make_int2(pos_x(q[i]), pos_y(q[i]) | zr);
+    if (a.errs) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a.errs[bi * 8 + i] = e[i];
+    }
+}
+
 }  // namespace zb
