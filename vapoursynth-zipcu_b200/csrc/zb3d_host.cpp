@@ -43,9 +43,7 @@ size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
 bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta);
 bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta);
 size_t batch_match_smem(const MatchArgs &m);
-size_t batch_filter_smem(bool final_);
-cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, size_t filter_smem,
-                         cudaStream_t st);
+cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st);
 cudaError_t filter_precision_init(int dev);
 size_t filter_precision_stack_floats(long long nblocks);
 cudaError_t launch_filter_precision(const FilterArgs &a, bool final_, float *stack, float *basic, float *weight,
@@ -1193,7 +1191,7 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
         a.status = d_status;
         a.wait_polls = wait_polls ? wait_polls : (1u << 22);
         a.unsatisfiable = unsatisfiable && g == (p.groups[0].empty() ? 1 : 0);
-        ce = launch_batch(a, g == 1, 0, 0, smem[g], batch_filter_smem(g == 1), st);
+        ce = launch_batch(a, g == 1, 0, 0, smem[g], st);
         for (int i = 0; i < (int)p.groups[g].size() && ce == cudaSuccess; ++i) {
             const BatchItem &it = p.groups[g][i];
             const Entry &en = *it.en;

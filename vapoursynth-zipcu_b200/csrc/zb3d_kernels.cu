@@ -6,7 +6,7 @@
 // the reference's operation order.
 //
 // Design (B200):
-//  * Filtering: 16 lanes per group (32 values each), the reference's transform order, FP32.
+//  * Filtering: 8 lanes per group, packed FP32x2 transforms (zb3d_filter.cuh).
 //  * Aggregation: signed 64-bit fixed point (2^32 = 1.0) with integer atomics,
 //    which is exact and order independent; the weight sum is accumulated once
 //    per patch at its origin and expanded by an 8x8 box sum in the finish pass.
@@ -16,21 +16,27 @@
 #include <cstdint>
 
 #include "zb3d_args.h"
+#include "zb3d_filter.cuh"
 #include "zb3d_match.cuh"
 #include "zb3d_match_scan.cuh"
 #include "zb3d_transforms.cuh"
 
 namespace zb {
 
+// The DCT in both dimensions: 2 warps of 4 groups per CTA (filter8_groups).
+template <bool FINAL>
+__global__ void __launch_bounds__(kFilter8Warps * 32) zb_filter8(FilterArgs a) {
+    __shared__ __align__(16) float sbuf[kFilterGroups * kGroupStride];
+    __shared__ __align__(16) float cbuf[FINAL ? kFilterGroups * kGroupStride : 4];  // Wiener coefficients
+    __shared__ long long offs[kFilterGroups * kOffStride];
+    filter8_groups<FINAL>(a, (long long)blockIdx.x * kFilterGroups, sbuf, cbuf, offs);
+}
+
 // ---------------------------------------------------------------------------
 // Collaborative filtering (vszipcu src/bm3d.cu:392-546) and aggregation into
 // signed 64-bit fixed point.
 // ---------------------------------------------------------------------------
 static constexpr int kFilterWarps = 4;
-
-__device__ __forceinline__ unsigned long long to_fix(float v) {
-    return (unsigned long long)__float2ll_rn(v * kFixScale);
-}
 
 // ---------------------------------------------------------------------------
 // Collaborative filtering with 16 lanes per group.  Lane (j, h), j = 0..7,
@@ -253,7 +259,7 @@ __device__ __forceinline__ void filter16_groups(const FilterArgs &a, long long g
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const float val = __fmaf_rn(w, d[p * 4 + t], E) - E;
-                atomicAdd(q + (2 * t + h) * a.pitch, to_fix(val));
+                atomicAdd(q + (2 * t + h) * a.pitch, to_fix(val * kFixScale));
             }
         }
         if (h == 0) {
@@ -262,7 +268,7 @@ __device__ __forceinline__ void filter16_groups(const FilterArgs &a, long long g
             const int2 v = a.list[grp * 8 + j];
             atomicAdd(a.den + pl * a.acc_plane_stride + ((unsigned)v.y >> 24) * a.acc_frame_stride +
                           (long long)(v.y & 0xffffff) * a.pitch + v.x,
-                      to_fix(wq));
+                      to_fix(wq * kFixScale));
         }
         __syncwarp(gm);  // the coefficient buffer is rewritten by the next plane
     }
@@ -379,11 +385,13 @@ __device__ __forceinline__ int batch_entry_of(const BatchArgs &b, long long item
 // items of the other kind are skipped, so two stream-ordered launches cover the list, each
 // kernel with the register budget of its own kind of work).
 // PHASE 1: the match tiles (kBatchMatchRows warps per CTA); PHASE 2: the filter chunks
-// (4 warps per CTA).  Each phase is one persistent launch with its own register budget.
+// (2 warps per CTA).  Each phase is one persistent launch with its own register budget.
 template <bool FINAL, int T2D, int T1D, int PHASE>
-__global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : 128) zb_batch(BatchArgs b) {
-    extern __shared__ __align__(16) float dyn[];  // matching tile, or the Wiener coefficient buffer
-    __shared__ float tbuf[PHASE == 1 ? 1 : kFilterWarps * 2 * kGroupBuf];
+__global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps * 32) zb_batch(BatchArgs b) {
+    extern __shared__ __align__(16) float dyn[];  // matching tile
+    __shared__ __align__(16) float sbuf[PHASE == 1 ? 4 : kFilterGroups * kGroupStride];
+    __shared__ __align__(16) float cbuf[PHASE == 1 || !FINAL ? 4 : kFilterGroups * kGroupStride];
+    __shared__ long long offs[PHASE == 1 ? 1 : kFilterGroups * kOffStride];
     __shared__ long long s_item;
     __shared__ int s_ok;
     static_assert(PHASE == 1 || PHASE == 2, "match phase or filter phase");
@@ -433,8 +441,8 @@ __global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : 128) zb_batch(B
             __threadfence();      // the count before the lists, for every reading thread
             const long long g0 = (item - E.first_filter) * kBatchGroups;
 #pragma unroll 1
-            for (int g = 0; g < kBatchGroups; g += 128 / 16)
-                filter16_groups<FINAL, T2D, T1D>(E.f, g0 + g, tbuf, dyn);
+            for (int g = 0; g < kBatchGroups && g0 + g < E.f.nblocks; g += kFilterGroups)
+                filter8_groups<FINAL>(E.f, g0 + g, sbuf, cbuf, offs);
         }
     }
 }
@@ -444,16 +452,22 @@ __global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : 128) zb_batch(B
 // ---------------------------------------------------------------------------
 template <bool FINAL, int T2D, int T1D>
 static cudaError_t launch_filter_t(const FilterArgs &a, cudaStream_t st) {
-    const long long threads = (long long)a.nblocks * 16;
-    const int tpb = kFilterWarps * 32;
-    const int dyn = FINAL ? (tpb / 16) * kCoeffBuf * (int)sizeof(float) : 0;  // Wiener coefficient buffer
-    auto k = zb_filter16<FINAL, T2D, T1D>;
-    if (FINAL) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
-        if (e != cudaSuccess) return e;
+    if constexpr (T2D == T_DCT && T1D == T_DCT) {
+        const unsigned grid = (unsigned)(((long long)a.nblocks + kFilterGroups - 1) / kFilterGroups);
+        zb_filter8<FINAL><<<grid, kFilter8Warps * 32, 0, st>>>(a);
+        return cudaGetLastError();
+    } else {
+        const long long threads = (long long)a.nblocks * 16;
+        const int tpb = kFilterWarps * 32;
+        const int dyn = FINAL ? (tpb / 16) * kCoeffBuf * (int)sizeof(float) : 0;  // Wiener coefficient buffer
+        auto k = zb_filter16<FINAL, T2D, T1D>;
+        if (FINAL) {
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+            if (e != cudaSuccess) return e;
+        }
+        k<<<(unsigned)((threads + tpb - 1) / tpb), tpb, dyn, st>>>(a);
+        return cudaGetLastError();
     }
-    k<<<(unsigned)((threads + tpb - 1) / tpb), tpb, dyn, st>>>(a);
-    return cudaGetLastError();
 }
 
 template <bool FINAL, int T2D>
@@ -503,10 +517,8 @@ cudaError_t launch_finish(const unsigned long long *num, const unsigned long lon
     return cudaGetLastError();
 }
 
-// Bytes of dynamic shared memory a batch entry needs: its matching tile (kBatchMatchRows
-// block rows), and the Wiener coefficient buffer of its filter chunks.
+// Bytes of dynamic shared memory a batch entry's matching needs (kBatchMatchRows block rows).
 size_t batch_match_smem(const MatchArgs &m) { return scan_smem_bytes(m, kBatchMatchRows); }
-size_t batch_filter_smem(bool final_) { return final_ ? (size_t)(128 / 16) * kCoeffBuf * sizeof(float) : 0; }
 
 template <class K>
 static cudaError_t launch_batch_k(K k, const BatchArgs &b, int threads, size_t smem, cudaStream_t st) {
@@ -528,16 +540,15 @@ static cudaError_t launch_batch_k(K k, const BatchArgs &b, int threads, size_t s
 // is built in (other kinds run entry by entry).  The match items and the filter items run as
 // two stream-ordered persistent launches (b.next must point at two counters); the filter
 // chunks still check, bounded, that their entry's matching is complete.
-// match_smem / filter_smem: dynamic shared memory of each kind of item.
-cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, size_t filter_smem,
-                         cudaStream_t st) {
+// match_smem: dynamic shared memory of the match items.
+cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st) {
     if (t2d != T_DCT || t1d != T_DCT) return cudaErrorNotSupported;
     cudaError_t e = launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 1> : zb_batch<false, T_DCT, T_DCT, 1>, b,
                                    kScanWarps * 32, match_smem, st);
     if (e != cudaSuccess) return e;
     b.next += 1;
-    return launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 2> : zb_batch<false, T_DCT, T_DCT, 2>, b, 128,
-                          filter_smem > 0 ? filter_smem : 16, st);
+    return launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 2> : zb_batch<false, T_DCT, T_DCT, 2>, b,
+                          kFilter8Warps * 32, 0, st);
 }
 
 }  // namespace zb
