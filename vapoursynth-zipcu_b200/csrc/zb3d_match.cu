@@ -412,6 +412,8 @@ size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta) {
 
 bool tc_eligible(const MatchArgs &a);                          // zb3d_match_tc.cu
 cudaError_t launch_match_tc(const MatchArgs &a, cudaStream_t st);
+bool temporal_rows_eligible(const MatchArgs &a, int metric);   // zb3d_match_temporal.cu
+cudaError_t launch_temporal_rows(const MatchArgs &a, cudaStream_t st);
 
 // The FP32 scan of the blocks the tensor-core kernel listed (SSD, radius 0).
 cudaError_t launch_tc_fallback(MatchArgs a, cudaStream_t st) {
@@ -463,7 +465,9 @@ cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_til
     }
     if (e != cudaSuccess) return e;
 temporal:
-    if (a.radius > 0) {
+    if (a.radius > 0 && temporal_rows_eligible(a, metric)) {
+        e = launch_temporal_rows(a, st);
+    } else if (a.radius > 0) {
         switch (metric) {
         case M_SSD: e = launch_temporal_m<M_SSD>(a, st); break;
         case M_SAD: e = launch_temporal_m<M_SAD>(a, st); break;

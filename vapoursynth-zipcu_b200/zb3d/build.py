@@ -2,7 +2,7 @@
 
     python -m zb3d.build        (from vapoursynth-zipcu_b200/)
 
-zb3d_kernels.cu, zb3d_match.cu and zb3d_match_tc.cu are compiled with -use_fast_math (the
+zb3d_kernels.cu, zb3d_match*.cu are compiled with -use_fast_math (the
 reference kernel's floating-point mode), zb3d_vagg.cu without it (IEEE sums and division, no
 flush-to-zero), the host in C++17; nvcc links them into one shared library.
 """
@@ -25,6 +25,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", f"-I{INCLUDE}
 UNITS = [
     ("zb3d_kernels.cu", ARCH + ["-use_fast_math"]),
     ("zb3d_match.cu", ARCH + ["-use_fast_math"]),
+    ("zb3d_match_temporal.cu", ARCH + ["-use_fast_math"]),
     ("zb3d_match_tc.cu", ARCH + ["-use_fast_math"]),
     ("zb3d_vagg.cu", ARCH),
     ("zb3d_pilot.cu", ARCH),
