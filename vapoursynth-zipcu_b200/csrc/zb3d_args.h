@@ -21,6 +21,11 @@ struct MatchArgs {
     int tiles_x;           // scan kernel: tiles per row; one more column of CTAs takes the clamped blocks
     int2 *list;            // [nby*nbx][8]: (x, y | z << 24)
     float *errs;           // [nby*nbx][8]: distances of the spatial list (radius > 0)
+    // Accumulators that start from zero after the matching (null: none): two arrays of
+    // zero_count 64-bit words.  The scan kernel writes the zeros itself, its stores being free
+    // beside the arithmetic; before the other matchers they are cleared by memset nodes.
+    unsigned long long *zero[2];
+    long long zero_count;
     int self_incl;         // 1: insert the block itself here (radius 0)
     int gen_mode;          // generic kernel: 0 = every block, 2 = the blocks listed in tc_ws
                            // (fallbacks of the tensor-core form)
@@ -66,11 +71,14 @@ struct BatchEntry {
     long long first_match, first_filter;  // first item number of each kind
 };
 
+// A kernel argument (about 20 KB): fields come from the constant bank, where no store of the
+// kernel makes the compiler load them again, and a captured launch carries its own copy.
+constexpr int kBatchEntries = 48;     // entries per work list; a larger batch has several
+
 struct BatchArgs {
-    const BatchEntry *entries;
+    BatchEntry entries[kBatchEntries];
     int nentries;
     long long match_total, items_total;   // match items, all items
-    unsigned long long *next;         // next item to take (starts at 0)
     unsigned *match_done;             // [nentries] match tiles finished
     int *status;                      // 0, or 1 when a filter chunk gave up waiting for its matching
     unsigned wait_polls;              // polls (about 0.1 us apart) before a wait gives up
@@ -80,7 +88,7 @@ struct BatchArgs {
 // Largest dynamic shared memory of a CTA on sm_100 (227 KB), less 1 KB for static variables.
 constexpr unsigned kSmemOptIn = 226 * 1024;
 
-constexpr int kBatchGroups = 128;     // groups per filter chunk
+constexpr int kBatchGroups = 32;      // groups per filter chunk
 constexpr int kBatchMatchRows = 8;    // block rows (warps) per match tile
 
 // Fixed-point scale of the accumulators: value * 2^32 held in a signed 64-bit sum.

@@ -25,6 +25,7 @@
 #include <tuple>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -43,7 +44,7 @@ size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
 bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta);
 bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta);
 size_t batch_match_smem(const MatchArgs &m);
-cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st);
+cudaError_t launch_batch(const BatchArgs &b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st);
 cudaError_t filter_precision_init(int dev);
 size_t filter_precision_stack_floats(long long nblocks);
 cudaError_t launch_filter_precision(const FilterArgs &a, bool final_, float *stack, float *basic, float *weight,
@@ -399,7 +400,8 @@ bool alloc_slot(Filter *f, Slot &s) {
 }
 
 // Block matching of one entry into the slot's match list.
-cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src) {
+// clear: the accumulators of the entry start from zero after it.
+cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, bool clear = false) {
         MatchArgs ma{};
         ma.frames = src;  // clip 0, plane 0: the matching plane of every window frame
         ma.fstride = (long long)en.plane_elems;
@@ -418,6 +420,11 @@ cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src) {
         ma.errs = f->radius > 0 ? s.errs : nullptr;
         ma.tc_ws = en.form == 1 ? s.tc_ws : nullptr;  // null: the FP32 scan
         ma.tc_stats = s.tc_stats;
+        if (clear) {
+            ma.zero[0] = s.num;
+            ma.zero[1] = s.den;
+            ma.zero_count = (long long)en.nplanes * f->tw * (long long)en.plane_elems;
+        }
         const int rows = en.rows;
         bool tiled = (en.bs == 4 || en.bs == 8);
         if (tiled) {
@@ -614,12 +621,14 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
         if (lo < best_ms) best_ms = lo;
         times.push_back({lo, cand});
     }
-    // the first candidate within 20% of the fastest: fewer block rows per CTA make one plane's
+    // The first candidate within 20% of the fastest: fewer block rows per CTA make one plane's
     // launch shorter by filling the GPU, but cost more in all (every range of candidate rows
     // builds a list of its own), which shows as soon as other streams fill it (640x480 at
-    // block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3 streams)
+    // block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3 streams).
+    // A plane that leaves SMs without a CTA even at one row takes the fastest.
+    const float slack = entry_scan_fits(e, 1) && scan_ctas(e, 1) > sms ? 1.2f : 1.0f;
     for (const auto &t : times)
-        if (bform < 0 && t.first <= 1.2f * best_ms) {
+        if (bform < 0 && t.first <= slack * best_ms) {
             bform = t.second.first;
             brows = t.second.second;
         }
@@ -738,11 +747,8 @@ cudaError_t run_entry_steps(Filter *f, Slot &s, const Entry &en, const float *sr
 cudaError_t run_entry(Filter *f, Slot &s, const Entry &en, const float *src, float *dst, bool basic) {
     cudaError_t e = cudaSuccess;
     {
-        const size_t acc = (size_t)en.nplanes * f->tw * en.plane_elems;
-        if ((e = cudaMemsetAsync(s.num, 0, acc * 8, s.st)) != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(s.den, 0, acc * 8, s.st)) != cudaSuccess) return e;
         if (f->profile) prof_event(f, f->prof_match, s.st);
-        if ((e = run_match(f, s, en, src)) != cudaSuccess) return e;
+        if ((e = run_match(f, s, en, src, true)) != cudaSuccess) return e;
         if (f->profile) prof_event(f, f->prof_match, s.st);
         FilterArgs fa{};
         fa.src = src;
@@ -927,14 +933,15 @@ namespace {
 struct BatchBuffers {
     char *arena = nullptr;
     size_t arena_bytes = 0;
-    BatchEntry *h_entries = nullptr;  // page-locked
-    size_t h_cap = 0;
     int *h_status = nullptr;          // page-locked
     cudaEvent_t ev_start = nullptr;   // the launching stream at the start of a batch
+    // One stream per held slot for the entries outside the work list, of the highest priority:
+    // their short dependent kernels run between the work list's CTAs instead of after them.
+    std::vector<cudaStream_t> streams;
 
     void release() {
+        for (cudaStream_t s : streams) cudaStreamDestroy(s);
         cudaFree(arena);
-        if (h_entries) cudaFreeHost(h_entries);
         if (h_status) cudaFreeHost(h_status);
         if (ev_start) cudaEventDestroy(ev_start);
         *this = BatchBuffers();
@@ -1016,10 +1023,10 @@ bool plan_batch(const zb3d_batch_job *jobs, int njobs, BatchPlan &p, char *err, 
             else p.fallback.push_back({j, &en});
         }
     }
-    // scratch layout: [counters | status | entries | lists | accumulators]
+    // scratch layout: [counters | status | lists | accumulators]
     p.nent = (int)(p.groups[0].size() + p.groups[1].size());
-    p.counters = align256(32 + 4 * (size_t)p.nent);
-    p.need = p.counters + 256 + align256(sizeof(BatchEntry) * (size_t)std::max(p.nent, 1));
+    p.counters = align256(4 * (size_t)std::max(p.nent, 1));
+    p.need = p.counters + 256;
     for (int g = 0; g < 2; ++g)
         for (const BatchItem &it : p.groups[g]) {
             p.list_off.push_back(p.need);
@@ -1047,24 +1054,33 @@ bool ensure_buffers(BatchBuffers &b, const BatchPlan &p, cudaStream_t st, char *
         }
         b.arena_bytes = p.need;
     }
-    if ((size_t)p.nent > b.h_cap || !b.h_status) {
-        cudaStreamSynchronize(st);
-        if (b.h_entries) cudaFreeHost(b.h_entries);
-        b.h_entries = nullptr;
-        b.h_cap = 0;
-        const size_t cap = std::max<size_t>(p.nent, 16);
-        if (cudaHostAlloc((void **)&b.h_entries, cap * sizeof(BatchEntry), cudaHostAllocDefault) != cudaSuccess ||
-            (!b.h_status && cudaHostAlloc((void **)&b.h_status, sizeof(int), cudaHostAllocDefault) != cudaSuccess)) {
-            cudaGetLastError();
-            set_err(err, errlen, "zb3d_process_batch: out of page-locked host memory.");
-            return false;
-        }
-        b.h_cap = cap;
+    if (!b.h_status && cudaHostAlloc((void **)&b.h_status, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        set_err(err, errlen, "zb3d_process_batch: out of page-locked host memory.");
+        return false;
     }
     if (!b.ev_start && cudaEventCreateWithFlags(&b.ev_start, cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
         set_err(err, errlen, "zb3d_process_batch: cannot create an event.");
         return false;
+    }
+    return true;
+}
+
+// A stream per filter with entries outside the work list.
+bool ensure_streams(BatchBuffers &b, const BatchPlan &p, char *err, size_t errlen) {
+    std::set<const void *> filters;
+    for (const BatchItem &it : p.fallback) filters.insert(p.jobs[it.job].filter);
+    int least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    while (b.streams.size() < filters.size()) {
+        cudaStream_t s = nullptr;
+        if (cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest) != cudaSuccess) {
+            cudaGetLastError();
+            set_err(err, errlen, "zb3d_process_batch: cannot create a stream.");
+            return false;
+        }
+        b.streams.push_back(s);
     }
     return true;
 }
@@ -1079,131 +1095,134 @@ std::map<Filter *, int> hold_slots(const BatchPlan &p) {
     return held;
 }
 
-void release_slots(std::map<Filter *, int> &held) {
-    for (auto &h : held) {
-        cudaStreamSynchronize(h.first->slots[h.second].st);
-        release_slot(h.first, h.second);
-    }
+void release_slots(std::map<Filter *, int> &held, BatchBuffers &b) {
+    for (cudaStream_t s : b.streams) cudaStreamSynchronize(s);
+    for (auto &h : held) release_slot(h.first, h.second);
     held.clear();
 }
 
 // The whole batch on `st`: entries outside the work list on the held slots' streams (after
 // what `st` holds so far, joined back at the end), the work-list launches and the finishes,
-// then the status word into b.h_status.  Builds the entry table in b.h_entries; with stream
-// capture the copy of that table is part of the graph and the table must stay as it is.
+// then the status word into b.h_status.
 cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *, int> &held, unsigned wait_polls,
                           int unsatisfiable, cudaStream_t st) {
     cudaError_t ce = cudaEventRecord(b.ev_start, st);
-    for (auto &h : held)
-        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(h.first->slots[h.second].st, b.ev_start, 0);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (ce == cudaSuccess) ce = cudaStreamIsCapturing(st, &capturing);
+    std::map<Filter *, Slot> slots;  // the held slots, on the batch's streams
+    for (auto &h : held) {
+        Slot s = h.first->slots[h.second];
+        const cudaStream_t own = s.st;
+        s.st = b.streams[slots.size()];
+        // after what the slot's own stream still holds (a captured batch has no such order)
+        if (ce == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
+            ce = cudaEventRecord(s.ev_up, own);
+            if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s.st, s.ev_up, 0);
+        }
+        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s.st, b.ev_start, 0);
+        slots.emplace(h.first, s);
+    }
     for (const BatchItem &it : p.fallback) {
         if (ce != cudaSuccess) break;
         Filter *f = reinterpret_cast<Filter *>(p.jobs[it.job].filter);
-        Slot &s = f->slots[held.at(f)];
-        ce = run_entry_steps(f, s, *it.en, p.jobs[it.job].d_src + it.en->src_off, p.jobs[it.job].d_dst + it.en->dst_off);
+        ce = run_entry_steps(f, slots.at(f), *it.en, p.jobs[it.job].d_src + it.en->src_off,
+                             p.jobs[it.job].d_dst + it.en->dst_off);
     }
     char *arena = b.arena;
-    unsigned long long *d_next = reinterpret_cast<unsigned long long *>(arena);  // [2][2]: group, kind
-    unsigned *d_done = reinterpret_cast<unsigned *>(arena + 32);                 // [nent]
+    unsigned *d_done = reinterpret_cast<unsigned *>(arena);  // [nent] match tiles finished
     int *d_status = reinterpret_cast<int *>(arena + p.counters);
-    BatchEntry *d_entries = reinterpret_cast<BatchEntry *>(arena + p.counters + 256);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(arena, 0, p.counters + 256, st);
-    // accumulators start at zero
-    if (ce == cudaSuccess && p.nent > 0) ce = cudaMemsetAsync(arena + p.acc_off[0], 0, p.need - p.acc_off[0], st);
-    size_t smem[2] = {0, 0};  // per group: matching tiles
-    long long totals[2][2] = {{0, 0}, {0, 0}};  // [group] (match items, all items)
+    // work lists of up to kBatchEntries entries of one filter kind
+    auto args = std::make_unique<BatchArgs>();
     int idx = 0;
-    for (int g = 0; g < 2 && ce == cudaSuccess; ++g) {
-        long long nm = 0;
-        const int first = idx;
-        for (const BatchItem &it : p.groups[g]) {
-            const Filter *f = reinterpret_cast<const Filter *>(p.jobs[it.job].filter);
-            const Entry &en = *it.en;
-            const float *src = p.jobs[it.job].d_src + en.src_off;
-            BatchEntry &B = b.h_entries[idx];
-            B = BatchEntry{};
-            int2 *list = reinterpret_cast<int2 *>(arena + p.list_off[idx]);
-            unsigned long long *num = reinterpret_cast<unsigned long long *>(arena + p.acc_off[idx]);
-            unsigned long long *den = reinterpret_cast<unsigned long long *>(
-                arena + p.acc_off[idx] + align256((size_t)en.nplanes * en.plane_elems * 8));
-            MatchArgs &m = B.m;
-            m.frames = src;  // clip 0, plane 0: the matching plane
-            m.fstride = (long long)en.plane_elems;
-            m.w = en.w;
-            m.h = en.h;
-            m.pitch = en.pitch;
-            m.bs = en.bs;
-            m.range = en.range;
-            m.nbx = en.nbx;
-            m.nby = en.nby;
-            m.nbx_al = en.nbx_al;
-            m.chunks = (2 * en.range + 1 + 3) / 4;
-            m.tile_pitch = 128 + 4 * m.chunks;
-            m.list = list;
-            m.self_incl = 1;
-            FilterArgs &fa = B.f;
-            fa.src = src;
-            fa.plane_stride = (long long)en.plane_elems;
-            fa.clip_stride = (long long)en.nplanes * fa.plane_stride;
-            fa.frame_stride = (long long)en.plane_elems;
-            fa.w = en.w;
-            fa.h = en.h;
-            fa.pitch = en.pitch;
-            fa.nplanes = en.nplanes;
-            fa.chroma = f->chroma;
-            fa.list = list;
-            fa.nblocks = (int)en.nblocks;
-            for (int i = 0; i < 3; ++i) fa.sigma[i] = en.sigma[i];
-            fa.extractor = f->extractor;
-            fa.num = num;
-            fa.den = den;
-            fa.acc_frame_stride = (long long)en.plane_elems;
-            fa.acc_plane_stride = (long long)en.plane_elems;
-            const int nbw = en.bs == 4 ? 31 : 16;
-            m.tiles_x = (en.nbx_al + nbw - 1) / nbw;
-            B.tiles_x = m.tiles_x + (en.nbx_al != en.nbx ? 1 : 0);
-            B.match_items = B.tiles_x * ((en.nby + kBatchMatchRows - 1) / kBatchMatchRows);
-            B.filter_items = (int)((en.nblocks + kBatchGroups - 1) / kBatchGroups);
-            B.first_match = nm;
-            nm += B.match_items;
-            smem[g] = std::max(smem[g], batch_match_smem(m));
-            ++idx;
+    bool testing = unsatisfiable != 0;
+    for (int g = 0; g < 2; ++g)
+        for (size_t at = 0; at < p.groups[g].size() && ce == cudaSuccess; at += kBatchEntries) {
+            const int n = (int)std::min<size_t>(kBatchEntries, p.groups[g].size() - at), base = idx;
+            size_t smem = 0;  // matching tiles
+            long long nm = 0;
+            for (int i = 0; i < n; ++i, ++idx) {
+                const BatchItem &it = p.groups[g][at + i];
+                const Filter *f = reinterpret_cast<const Filter *>(p.jobs[it.job].filter);
+                const Entry &en = *it.en;
+                const float *src = p.jobs[it.job].d_src + en.src_off;
+                BatchEntry &B = args->entries[i];
+                B = BatchEntry{};
+                int2 *list = reinterpret_cast<int2 *>(arena + p.list_off[idx]);
+                unsigned long long *num = reinterpret_cast<unsigned long long *>(arena + p.acc_off[idx]);
+                unsigned long long *den = reinterpret_cast<unsigned long long *>(
+                    arena + p.acc_off[idx] + align256((size_t)en.nplanes * en.plane_elems * 8));
+                MatchArgs &m = B.m;
+                m.frames = src;  // clip 0, plane 0: the matching plane
+                m.fstride = (long long)en.plane_elems;
+                m.w = en.w;
+                m.h = en.h;
+                m.pitch = en.pitch;
+                m.bs = en.bs;
+                m.range = en.range;
+                m.nbx = en.nbx;
+                m.nby = en.nby;
+                m.nbx_al = en.nbx_al;
+                m.chunks = (2 * en.range + 1 + 3) / 4;
+                m.tile_pitch = 128 + 4 * m.chunks;
+                m.list = list;
+                m.self_incl = 1;
+                m.zero[0] = num;  // cleared by the match items, which the filter chunks wait for
+                m.zero[1] = den;
+                m.zero_count = (long long)en.nplanes * (long long)en.plane_elems;
+                FilterArgs &fa = B.f;
+                fa.src = src;
+                fa.plane_stride = (long long)en.plane_elems;
+                fa.clip_stride = (long long)en.nplanes * fa.plane_stride;
+                fa.frame_stride = (long long)en.plane_elems;
+                fa.w = en.w;
+                fa.h = en.h;
+                fa.pitch = en.pitch;
+                fa.nplanes = en.nplanes;
+                fa.chroma = f->chroma;
+                fa.list = list;
+                fa.nblocks = (int)en.nblocks;
+                for (int i = 0; i < 3; ++i) fa.sigma[i] = en.sigma[i];
+                fa.extractor = f->extractor;
+                fa.num = num;
+                fa.den = den;
+                fa.acc_frame_stride = (long long)en.plane_elems;
+                fa.acc_plane_stride = (long long)en.plane_elems;
+                const int nbw = en.bs == 4 ? 31 : 16;
+                m.tiles_x = (en.nbx_al + nbw - 1) / nbw;
+                B.tiles_x = m.tiles_x + (en.nbx_al != en.nbx ? 1 : 0);
+                B.match_items = B.tiles_x * ((en.nby + kBatchMatchRows - 1) / kBatchMatchRows);
+                B.filter_items = (int)((en.nblocks + kBatchGroups - 1) / kBatchGroups);
+                B.first_match = nm;
+                nm += B.match_items;
+                smem = std::max(smem, batch_match_smem(m));
+            }
+            long long nf = nm;
+            for (int i = 0; i < n; ++i) {
+                args->entries[i].first_filter = nf;
+                nf += args->entries[i].filter_items;
+            }
+            args->nentries = n;
+            args->match_total = nm;
+            args->items_total = nf;
+            args->match_done = d_done + base;
+            args->status = d_status;
+            args->wait_polls = wait_polls ? wait_polls : (1u << 22);
+            args->unsatisfiable = testing;
+            testing = false;  // the first entry of the batch only
+            ce = launch_batch(*args, g == 1, 0, 0, smem, st);
+            for (int i = 0; i < n && ce == cudaSuccess; ++i) {
+                const BatchItem &it = p.groups[g][at + i];
+                const Entry &en = *it.en;
+                const FilterArgs &fa = args->entries[i].f;
+                ce = launch_finish(fa.num, fa.den, fa.acc_plane_stride, fa.acc_frame_stride, en.w, en.h, en.pitch,
+                                   en.nplanes, 1, en.proc_mask, p.jobs[it.job].d_dst + en.dst_off, en.pitch,
+                                   (long long)en.plane_elems, 0, st);
+            }
         }
-        long long nf = nm;
-        for (int i = first; i < idx; ++i) {
-            b.h_entries[i].first_filter = nf;
-            nf += b.h_entries[i].filter_items;
-        }
-        totals[g][0] = nm;
-        totals[g][1] = nf;
-    }
-    if (ce == cudaSuccess && p.nent > 0)
-        ce = cudaMemcpyAsync(d_entries, b.h_entries, sizeof(BatchEntry) * (size_t)p.nent, cudaMemcpyHostToDevice, st);
-    for (int g = 0, base = 0; g < 2 && ce == cudaSuccess; base += (int)p.groups[g].size(), ++g) {
-        if (p.groups[g].empty()) continue;
-        BatchArgs a{};
-        a.entries = d_entries + base;
-        a.nentries = (int)p.groups[g].size();
-        a.match_total = totals[g][0];
-        a.items_total = totals[g][1];
-        a.next = d_next + 2 * g;
-        a.match_done = d_done + base;
-        a.status = d_status;
-        a.wait_polls = wait_polls ? wait_polls : (1u << 22);
-        a.unsatisfiable = unsatisfiable && g == (p.groups[0].empty() ? 1 : 0);
-        ce = launch_batch(a, g == 1, 0, 0, smem[g], st);
-        for (int i = 0; i < (int)p.groups[g].size() && ce == cudaSuccess; ++i) {
-            const BatchItem &it = p.groups[g][i];
-            const Entry &en = *it.en;
-            const BatchEntry &B = b.h_entries[base + i];
-            ce = launch_finish(B.f.num, B.f.den, B.f.acc_plane_stride, B.f.acc_frame_stride, en.w, en.h, en.pitch,
-                               en.nplanes, 1, en.proc_mask, p.jobs[it.job].d_dst + en.dst_off, en.pitch,
-                               (long long)en.plane_elems, 0, st);
-        }
-    }
-    for (auto &h : held) {
+    for (auto &h : slots) {
         if (ce != cudaSuccess) break;
-        Slot &s = h.first->slots[h.second];
+        const Slot &s = h.second;
         ce = cudaEventRecord(s.ev_up, s.st);
         if (ce == cudaSuccess) ce = cudaStreamWaitEvent(st, s.ev_up, 0);
     }
@@ -1684,12 +1703,12 @@ int zb3d_process_batch_ex(const zb3d_batch_job *jobs, int njobs, void *stream, u
     const cudaStream_t st = (cudaStream_t)stream;
     BatchCtx &ctx = batch_ctx(p.device);
     std::lock_guard<std::mutex> lk(ctx.mu);
-    if (!ensure_buffers(ctx.buf, p, st, err, errlen)) return -1;
+    if (!ensure_buffers(ctx.buf, p, st, err, errlen) || !ensure_streams(ctx.buf, p, err, errlen)) return -1;
     std::map<Filter *, int> held = hold_slots(p);
     cudaError_t ce = enqueue_batch(p, ctx.buf, held, wait_polls, unsatisfiable, st);
     const cudaError_t cs = cudaStreamSynchronize(st);
     if (ce == cudaSuccess) ce = cs;
-    release_slots(held);
+    release_slots(held, ctx.buf);
     if (ce != cudaSuccess) {
         set_err(err, errlen, "zb3d_process_batch: %s.", cudaGetErrorString(ce));
         return -1;
@@ -1722,7 +1741,7 @@ zb3d_batch *zb3d_batch_create(const zb3d_batch_job *jobs, int njobs, char *err, 
         cudaGetLastError();
         set_err(err, errlen, "zb3d_batch_create: %s (%s).", what, cudaGetErrorString(e));
         if (b->cap) cudaStreamSynchronize(b->cap);
-        release_slots(b->held);
+        release_slots(b->held, b->buf);
         if (b->exec) cudaGraphExecDestroy(b->exec);
         if (b->cap) cudaStreamDestroy(b->cap);
         b->buf.release();
@@ -1730,7 +1749,7 @@ zb3d_batch *zb3d_batch_create(const zb3d_batch_job *jobs, int njobs, char *err, 
     };
     cudaError_t e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
     if (e != cudaSuccess) return fail("cannot create a stream", e);
-    if (!ensure_buffers(b->buf, b->plan, b->cap, err, errlen)) {
+    if (!ensure_buffers(b->buf, b->plan, b->cap, err, errlen) || !ensure_streams(b->buf, b->plan, err, errlen)) {
         cudaStreamDestroy(b->cap);
         b->buf.release();
         return nullptr;
@@ -1785,7 +1804,7 @@ void zb3d_batch_free(zb3d_batch *b) {
     if (b->cap) cudaStreamSynchronize(b->cap);
     cudaDeviceSynchronize();  // replays may still run on the callers' streams
     if (b->exec) cudaGraphExecDestroy(b->exec);
-    zb::release_slots(b->held);
+    zb::release_slots(b->held, b->buf);
     if (b->cap) cudaStreamDestroy(b->cap);
     b->buf.release();
     delete b;

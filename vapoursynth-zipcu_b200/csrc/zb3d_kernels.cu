@@ -300,75 +300,110 @@ struct FinishArgs {
     int mode;
 };
 
-// One CTA per 32 x 32 output pixels of one plane (and frame slot): the 39 x 39 tile of
-// origin weights that their 8x8 boxes cover is read once into shared memory, summed along
-// rows (8 wide), then each thread slides an 8-row sum down its column for 4 pixels.  The
-// sums are int64, exact in any order.
-constexpr int kFinishRows = 32;
+// One warp per strip of 56 output columns and `rows` output rows (a multiple of 8).  A lane
+// owns two neighbouring columns (16-byte loads; 8 columns to the left of the strip are read for
+// their weights only) and walks down them in chunks of 8 rows, all of whose loads are in
+// flight together: the 8-row sum of origin weights of a column slides in registers, and the
+// 8-column sum over it comes from three exchanges between lanes.  The sums are int64, exact in
+// any order.  No shared memory and no barrier: the kernel moves 16 B + 4 or 8 B per pixel and
+// is bound by that.  (A 39 x 39 tile of weights in shared memory summed per pixel, the form
+// before: @@FIN@@)
+constexpr int kFinishCols = 56;
+constexpr int kFinishWarps = 4;
 
-__global__ void __launch_bounds__(256) zb_finish(FinishArgs a) {
-    constexpr int TR = kFinishRows + 7, TC = 32 + 7;
-    __shared__ long long t[TR][TC + 1];
-    __shared__ long long hs[TR][32];
+__device__ __forceinline__ longlong2 finish_load(const unsigned long long *row, int x, int w, bool vec) {
+    longlong2 v = make_longlong2(0, 0);
+    if (x < 0 || x >= w) return v;
+    if (vec && x + 1 < w) return *reinterpret_cast<const longlong2 *>(row + x);
+    v.x = (long long)row[x];
+    if (x + 1 < w) v.y = (long long)row[x + 1];
+    return v;
+}
+
+// vec: rows of the accumulators start on 16 bytes (an even pitch); vec_out: pairs of output
+// pixels on 8 bytes.
+__global__ void __launch_bounds__(kFinishWarps * 32) zb_finish(FinishArgs a, int rows, bool vec, bool vec_out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int plane = blockIdx.z / a.tw, slot = blockIdx.z - plane * a.tw;
     if (!((a.proc_mask >> plane) & 1)) return;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * kFinishRows;
+    const int xs = (blockIdx.x * kFinishWarps + warp) * kFinishCols;
+    if (xs >= a.w) return;
+    const int x = xs - 8 + 2 * lane, y0 = blockIdx.y * rows;
     const long long base = plane * a.acc_plane_stride + slot * a.acc_frame_stride;
-    const unsigned long long *den = a.den + base;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
-    constexpr int PER = kFinishRows / 8;  // output rows per thread
-    const int x = x0 + threadIdx.x;
-    const int ry = threadIdx.y * PER;     // first tile row of this thread's pixels
-    long long ns[PER];                    // this thread's numerators, loaded before the tile
+    const unsigned long long *num = a.num + base, *den = a.den + base;
+    const bool out = lane >= 4 && x < a.w;
+    float *o = a.dst + plane * a.dst_plane_stride + (a.mode ? (long long)slot * 2 * a.h * a.dst_pitch : 0);
+    const long long second = (long long)a.h * a.dst_pitch;  // mode 1: the weights' plane
+    longlong2 prev[8];
+    long long sa = 0, sb = 0;  // 8-row sums of the two columns
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int y = y0 + ry + i;
-        ns[i] = (x < a.w && y < a.h) ? (long long)a.num[base + (long long)y * a.pitch + x] : 0;
+    for (int k = 0; k < 8; ++k) {
+        const int y = y0 - 8 + k;
+        prev[k] = y >= 0 ? finish_load(den + (long long)y * a.pitch, x, a.w, vec) : make_longlong2(0, 0);
     }
-    for (int i = tid; i < TR * TC; i += 256) {
-        const int r = i / TC, c = i - r * TC;
-        const int gy = y0 - 7 + r, gx = x0 - 7 + c;
-        t[r][c] = (gy >= 0 && gy < a.h && gx >= 0 && gx < a.w) ? (long long)den[(long long)gy * a.pitch + gx] : 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        sa += prev[k].x;
+        sb += prev[k].y;
     }
-    __syncthreads();
-    for (int i = tid; i < TR * 32; i += 256) {
-        const int r = i >> 5, c = i & 31;
-        long long s = 0;
+    const int yend = min(y0 + rows, a.h);
+    for (int yc = y0; yc < yend; yc += 8) {
+        longlong2 cur[8], n[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) s += t[r][c + k];
-        hs[r][c] = s;
-    }
-    __syncthreads();
-    if (x >= a.w) return;
-    long long ds = 0;
+        for (int k = 0; k < 8; ++k) {
+            const int y = min(yc + k, a.h - 1);
+            cur[k] = finish_load(den + (long long)y * a.pitch, x, a.w, vec);
+            n[k] = out ? finish_load(num + (long long)y * a.pitch, x, a.w, vec) : make_longlong2(0, 0);
+        }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) ds += hs[ry + k][threadIdx.x];
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        const int y = y0 + ry + i;
-        if (y >= a.h) return;
-        if (i > 0) ds += hs[ry + i + 7][threadIdx.x] - hs[ry + i - 1][threadIdx.x];
-        const float nf = __ll2float_rn(ns[i]) * kFixInv;
-        const float df = __ll2float_rn(ds) * kFixInv;
-        if (a.mode == 0) {
-            a.dst[plane * a.dst_plane_stride + (long long)y * a.dst_pitch + x] = __fdiv_rn(nf, df);
-        } else {
-            float *o = a.dst + plane * a.dst_plane_stride + (long long)slot * 2 * a.h * a.dst_pitch;
-            o[(long long)y * a.dst_pitch + x] = nf;
-            o[(long long)(a.h + y) * a.dst_pitch + x] = df;
+        for (int k = 0; k < 8; ++k) {
+            const int y = yc + k;
+            sa += cur[k].x - prev[k].x;
+            sb += cur[k].y - prev[k].y;
+            prev[k] = cur[k];
+            // columns x - 6 .. x + 1, and x - 7 .. x
+            long long wb = sa + sb;
+            wb += __shfl_up_sync(0xffffffffu, wb, 1);
+            wb += __shfl_up_sync(0xffffffffu, wb, 2);
+            const long long wa = wb - sb + __shfl_up_sync(0xffffffffu, sb, 4);
+            if (!out || y >= yend) continue;
+            const float na = __ll2float_rn(n[k].x) * kFixInv, nb = __ll2float_rn(n[k].y) * kFixInv;
+            const float da = __ll2float_rn(wa) * kFixInv, db = __ll2float_rn(wb) * kFixInv;
+            float *row = o + (long long)y * a.dst_pitch + x;
+            if (a.mode == 0) {
+                const float2 v = make_float2(__fdiv_rn(na, da), __fdiv_rn(nb, db));
+                if (vec_out && x + 1 < a.w) {
+                    *reinterpret_cast<float2 *>(row) = v;
+                } else {
+                    row[0] = v.x;
+                    if (x + 1 < a.w) row[1] = v.y;
+                }
+            } else if (vec_out && x + 1 < a.w) {
+                *reinterpret_cast<float2 *>(row) = make_float2(na, nb);
+                *reinterpret_cast<float2 *>(row + second) = make_float2(da, db);
+            } else {
+                row[0] = na;
+                row[second] = da;
+                if (x + 1 < a.w) {
+                    row[1] = nb;
+                    row[second + 1] = db;
+                }
+            }
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Batch: one persistent launch over a work list of several plane entries (of any sizes)
-// that share the filter kind.  CTAs of 128 threads take items in order from a global
-// counter: every match tile of every entry, then every filter chunk.  A filter chunk of an
-// entry waits until all of that entry's match tiles are done (a bounded spin on its
-// counter; on timeout the chunk is skipped and the status word set).  Match items never
-// wait, and every item a CTA waits on was taken earlier by a running CTA, so the list
-// always drains.  Lists are written and read within the launch with ordinary loads and a
-// fence on both sides of the counter.
+// Batch: two launches over a work list of several plane entries (of any sizes) that share the
+// filter kind, one CTA per item: the match tiles of every entry, then the filter chunks of
+// every entry.  A filter chunk checks, bounded, that all of its entry's match tiles are done
+// (the launches are stream-ordered, so they are; on timeout the chunk is skipped and the
+// status word set, and the chunks after it do not wait).  Lists are written and read with
+// ordinary loads and a fence on both sides of the counter.
+// Items go to CTAs in order, so those in flight are neighbours in a plane and share its
+// lines, and the CTAs of a higher-priority stream get their turn between them.  (Persistent
+// CTAs taking chunks of 128 groups from a counter kept the entries outside the list waiting for
+// whole phases, and spread the chunks in flight over a third of a 4K plane: @@BAT@@)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int batch_entry_of(const BatchArgs &b, long long item, bool filter) {
     int lo = 0, hi = b.nentries - 1;  // last entry whose first item <= item
@@ -381,69 +416,59 @@ __device__ __forceinline__ int batch_entry_of(const BatchArgs &b, long long item
     return lo;
 }
 
-// PHASE 0: the whole list in one launch; 1: match items only; 2: filter items only (the
-// items of the other kind are skipped, so two stream-ordered launches cover the list, each
-// kernel with the register budget of its own kind of work).
-// PHASE 1: the match tiles (kBatchMatchRows warps per CTA); PHASE 2: the filter chunks
-// (2 warps per CTA).  Each phase is one persistent launch with its own register budget.
-template <bool FINAL, int T2D, int T1D, int PHASE>
-__global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps * 32) zb_batch(BatchArgs b) {
+// PHASE 1: a match tile (8 warps); PHASE 2: a filter chunk (2 warps).
+template <bool FINAL, int PHASE>
+__global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps * 32) zb_batch(const __grid_constant__ BatchArgs b) {
     extern __shared__ __align__(16) float dyn[];  // matching tile
     __shared__ __align__(16) float sbuf[PHASE == 1 ? 4 : kFilterGroups * kGroupStride];
     __shared__ __align__(16) float cbuf[PHASE == 1 || !FINAL ? 4 : kFilterGroups * kGroupStride];
     __shared__ long long offs[PHASE == 1 ? 1 : kFilterGroups * kOffStride];
-    __shared__ long long s_item;
     __shared__ int s_ok;
     static_assert(PHASE == 1 || PHASE == 2, "match phase or filter phase");
-    const long long first = PHASE == 2 ? b.match_total : 0;
-    const long long last = PHASE == 1 ? b.match_total : b.items_total;
-    for (;;) {
-        __syncthreads();  // the previous item is done with shared memory
-        if (threadIdx.x == 0) s_item = first + (long long)atomicAdd(b.next, 1ull);
-        __syncthreads();
-        const long long item = s_item;
-        if (item >= last) break;
-        if constexpr (PHASE == 1) {
-            const int e = batch_entry_of(b, item, false);
-            const BatchEntry &E = b.entries[e];
-            const int local = (int)(item - E.first_match);
-            const int bx = local % E.tiles_x, by = local / E.tiles_x;
-            if (bx == E.m.tiles_x) {  // the clamped last block column
-                const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
-                if (cy < E.m.nby) column_block<M_SSD>(E.m, cy);
-            } else if (E.m.bs == 4) {
-                scan_tile<M_SSD, true, 4>(E.m, bx, by, kBatchMatchRows, dyn);
-            } else {
-                scan_tile<M_SSD, false, 8>(E.m, bx, by, kBatchMatchRows, dyn);
-            }
-            __threadfence();  // each thread's list stores before the tile's count
-            __syncthreads();
-            if (threadIdx.x == 0) atomicAdd(&b.match_done[e], 1u);
+    const long long item = (PHASE == 2 ? b.match_total : 0) + blockIdx.x;
+    if constexpr (PHASE == 1) {
+        const int e = batch_entry_of(b, item, false);
+        const BatchEntry &E = b.entries[e];
+        const MatchArgs &m = E.m;
+        const int local = (int)(item - E.first_match);
+        const int bx = local % E.tiles_x, by = local / E.tiles_x;
+        zero_slice(m.zero, m.zero_count, local, E.match_items);
+        if (bx == m.tiles_x) {  // the clamped last block column
+            const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
+            if (cy < m.nby) column_block<M_SSD>(m, cy);
+        } else if (m.bs == 4) {
+            scan_tile<M_SSD, true, 4>(m, bx, by, kBatchMatchRows, dyn);
         } else {
-            const int e = batch_entry_of(b, item, true);
-            const BatchEntry &E = b.entries[e];
-            if (threadIdx.x == 0) {
-                const unsigned need = (unsigned)E.match_items + ((b.unsatisfiable && e == 0) ? 1u : 0u);
-                volatile unsigned *done = b.match_done + e;
-                int ok = 0;
-                for (unsigned i = 0; i < b.wait_polls; ++i) {
-                    if (*done >= need) {
-                        ok = 1;
-                        break;
-                    }
-                    __nanosleep(100);
-                }
-                if (!ok) atomicCAS(b.status, 0, 1);
-                s_ok = ok;
-            }
-            __syncthreads();
-            if (!s_ok) continue;  // this chunk is left out; the status tells the host
-            __threadfence();      // the count before the lists, for every reading thread
-            const long long g0 = (item - E.first_filter) * kBatchGroups;
-#pragma unroll 1
-            for (int g = 0; g < kBatchGroups && g0 + g < E.f.nblocks; g += kFilterGroups)
-                filter8_groups<FINAL>(E.f, g0 + g, sbuf, cbuf, offs);
+            scan_tile<M_SSD, false, 8>(m, bx, by, kBatchMatchRows, dyn);
         }
+        __threadfence();  // each thread's list stores before the tile's count
+        __syncthreads();
+        if (threadIdx.x == 0) atomicAdd(&b.match_done[e], 1u);
+    } else {
+        const int e = batch_entry_of(b, item, true);
+        const BatchEntry &E = b.entries[e];
+        if (threadIdx.x == 0) {
+            const unsigned need = (unsigned)E.match_items + ((b.unsatisfiable && e == 0) ? 1u : 0u);
+            volatile unsigned *done = b.match_done + e;
+            int ok = 0;
+            for (unsigned i = 0; i < b.wait_polls && *(volatile int *)b.status == 0; ++i) {
+                if (*done >= need) {
+                    ok = 1;
+                    break;
+                }
+                __nanosleep(100);
+            }
+            if (!ok) atomicCAS(b.status, 0, 1);
+            s_ok = ok;
+        }
+        __syncthreads();
+        if (!s_ok) return;  // this chunk is left out; the status tells the host
+        __threadfence();      // the count before the lists, for every reading thread
+        const FilterArgs &f = E.f;
+        const long long g0 = (item - E.first_filter) * kBatchGroups;
+#pragma unroll 1
+        for (int g = 0; g < kBatchGroups && g0 + g < f.nblocks; g += kFilterGroups)
+            filter8_groups<FINAL>(f, g0 + g, sbuf, cbuf, offs);
     }
 }
 
@@ -512,8 +537,15 @@ cudaError_t launch_finish(const unsigned long long *num, const unsigned long lon
     a.dst_pitch = dst_pitch;
     a.dst_plane_stride = dst_plane_stride;
     a.mode = mode;
-    dim3 grid((w + 31) / 32, (h + kFinishRows - 1) / kFinishRows, nplanes * a.tw);
-    zb_finish<<<grid, dim3(32, 8), 0, st>>>(a);
+    const int strips = (w + kFinishCols - 1) / kFinishCols, planes = nplanes * a.tw;
+    // 32 rows read 25% more weights than pixels, 8 rows 100%: fewer rows only where 32 would
+    // leave warps missing (16 fit an SM)
+    const int rows = (long long)strips * ((h + 31) / 32) * planes >= 148 * 16 ? 32 : 8;
+    const bool vec = pitch % 2 == 0 && acc_plane_stride % 2 == 0 && acc_frame_stride % 2 == 0 &&
+                     reinterpret_cast<uintptr_t>(num) % 16 == 0 && reinterpret_cast<uintptr_t>(den) % 16 == 0;
+    const bool vec_out = dst_pitch % 2 == 0 && dst_plane_stride % 2 == 0 && reinterpret_cast<uintptr_t>(dst) % 8 == 0;
+    dim3 grid((strips + kFinishWarps - 1) / kFinishWarps, (h + rows - 1) / rows, planes);
+    zb_finish<<<grid, kFinishWarps * 32, 0, st>>>(a, rows, vec, vec_out);
     return cudaGetLastError();
 }
 
@@ -521,33 +553,28 @@ cudaError_t launch_finish(const unsigned long long *num, const unsigned long lon
 size_t batch_match_smem(const MatchArgs &m) { return scan_smem_bytes(m, kBatchMatchRows); }
 
 template <class K>
-static cudaError_t launch_batch_k(K k, const BatchArgs &b, int threads, size_t smem, cudaStream_t st) {
+static cudaError_t launch_batch_k(K k, const BatchArgs &b, long long items, int threads, size_t smem,
+                                  cudaStream_t st) {
+    if (items <= 0) return cudaSuccess;
     // the same limit at every launch (see launch_scan_t), less the static buffers
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, k);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemOptIn - fa.sharedSizeBytes));
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, smem) != cudaSuccess || per < 1) per = 1;
-    k<<<sms * per, threads, smem, st>>>(b);
+    k<<<(unsigned)items, threads, smem, st>>>(b);
     return cudaGetLastError();
 }
 
 // The batch kernels for the filter kind (final, t2d, t1d); only the DCT in both dimensions
-// is built in (other kinds run entry by entry).  The match items and the filter items run as
-// two stream-ordered persistent launches (b.next must point at two counters); the filter
-// chunks still check, bounded, that their entry's matching is complete.
-// match_smem: dynamic shared memory of the match items.
-cudaError_t launch_batch(BatchArgs b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st) {
+// is built in (other kinds run entry by entry).  match_smem: dynamic shared memory of the
+// match items.
+cudaError_t launch_batch(const BatchArgs &b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st) {
     if (t2d != T_DCT || t1d != T_DCT) return cudaErrorNotSupported;
-    cudaError_t e = launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 1> : zb_batch<false, T_DCT, T_DCT, 1>, b,
-                                   kScanWarps * 32, match_smem, st);
+    cudaError_t e = launch_batch_k(final_ ? zb_batch<true, 1> : zb_batch<false, 1>, b, b.match_total, kScanWarps * 32,
+                                   match_smem, st);
     if (e != cudaSuccess) return e;
-    b.next += 1;
-    return launch_batch_k(final_ ? zb_batch<true, T_DCT, T_DCT, 2> : zb_batch<false, T_DCT, T_DCT, 2>, b,
+    return launch_batch_k(final_ ? zb_batch<true, 2> : zb_batch<false, 2>, b, b.items_total - b.match_total,
                           kFilter8Warps * 32, 0, st);
 }
 

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(128) zb_match_column(MatchArgs a) {
 template <int M, bool SHARED, int BS>
 __global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a, int rows) {
     extern __shared__ __align__(16) float tile[];
+    zero_slice(a.zero, a.zero_count, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
     if ((int)blockIdx.x == a.tiles_x) {
         const int warp = threadIdx.x >> 5, by = blockIdx.y * rows + warp;
         if (warp < rows && by < a.nby) column_block<M>(a, by);
@@ -426,7 +427,15 @@ cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_til
     cudaError_t e = cudaSuccess;
     const bool tiled = use_tiled && (a.bs == 4 || a.bs == 8);
     a.self_incl = a.radius == 0;
-    if (metric == M_SSD && a.tc_ws != nullptr && tc_eligible(a)) {
+    const bool tc = metric == M_SSD && a.tc_ws != nullptr && tc_eligible(a);
+    a.chunks = (2 * a.range + 1 + 3) / 4;
+    a.tile_pitch = 128 + 4 * a.chunks;
+    if (a.zero[0] && (tc || !tiled || !scan_rows(a, metric, rows_per_cta))) {
+        for (int k = 0; k < 2; ++k)
+            if ((e = cudaMemsetAsync(a.zero[k], 0, (size_t)a.zero_count * 8, st)) != cudaSuccess) return e;
+        a.zero[0] = nullptr;
+    }
+    if (tc) {
         // tensor-core bound + exact re-rank; the blocks it lists get the FP32 scan
         if ((e = launch_match_tc(a, st)) != cudaSuccess) return e;
         a.gen_mode = 2;
@@ -434,8 +443,6 @@ cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_til
         goto temporal;
     }
     if (tiled) {
-        a.chunks = (2 * a.range + 1 + 3) / 4;
-        a.tile_pitch = 128 + 4 * a.chunks;
         switch (metric) {
         case M_SSD: e = launch_tiled_m<M_SSD>(a, rows_per_cta, st); break;
         case M_SAD: e = launch_tiled_m<M_SAD>(a, rows_per_cta, st); break;

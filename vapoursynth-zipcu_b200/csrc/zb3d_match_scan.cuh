@@ -56,9 +56,9 @@ __device__ __forceinline__ float2 f4hi(const float4 &v) { return make_float2(v.z
 // (strict less), so the list is the one of immediate insertion.  Slot i of lane l is at
 // 256 i + 8 l bytes: whatever slots the lanes are at, a half warp touches 32 banks.
 // ---------------------------------------------------------------------------
-constexpr int kPend = 8;                        // slots per lane
+constexpr int kPend = 16;                       // slots per lane
 constexpr int kPendBytes = kPend * 32 * 8;      // per warp
-constexpr int kPendFull = (kPend - 4) * 256;    // a step appends at most 4
+constexpr int kPendFull = (kPend - 8) * 256;    // two steps append at most 8
 
 __device__ __forceinline__ void pend_store(unsigned at, float err, int pos) {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "f"(err), "r"(pos) : "memory");
@@ -186,6 +186,26 @@ __device__ __forceinline__ void scan_step_append(const float *pc, int pp, int g,
     if (__any_sync(kFull, end > base + kPendFull)) pend_drain(base, end, e, q);
 }
 
+// Two whole steps with one vote.
+template <int M, bool SHARED, int GF>
+__device__ __forceinline__ void scan_two_steps(const float *pc, int pp, int g, const float2 (&nc)[4][4],
+                                               float (&st)[4], int pos, unsigned base, unsigned &end, float (&e)[8],
+                                               int (&q)[8]) {
+    float err[2][4];
+    scan_step<M, GF, false, 3>(pc, pp, g, nc, st, err[0]);
+    scan_step<M, GF, false, 3>(pc + 4, pp, g, nc, st, err[1]);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        err[c >> 2][c & 3] += SHARED ? __shfl_down_sync(kFull, err[c >> 2][c & 3], 1) : __shfl_xor_sync(kFull, err[c >> 2][c & 3], 1);
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        if (err[c >> 2][c & 3] < e[7]) {
+            pend_store(end, err[c >> 2][c & 3], pos + c);
+            end += 256;
+        }
+    if (__any_sync(kFull, end > base + kPendFull)) pend_drain(base, end, e, q);
+}
+
 // Bytes of dynamic shared memory: the two copies of the tile, then the queues.
 inline size_t scan_tile_bytes(const MatchArgs &a, int rows_per_cta) {
     return (size_t)((rows_per_cta - 1) * a.bs + 2 * a.range + 8) * 8 * tile2_g(a.tile_pitch, tile2_fixed(a.chunks)) *
@@ -194,6 +214,20 @@ inline size_t scan_tile_bytes(const MatchArgs &a, int rows_per_cta) {
 
 inline size_t scan_smem_bytes(const MatchArgs &a, int rows_per_cta) {
     return scan_tile_bytes(a, rows_per_cta) + (size_t)kScanWarps * kPendBytes;
+}
+
+// CTA `part` of `parts` clears its share of the accumulators (16-byte stores; the arrays start
+// on 16 bytes).
+__device__ __forceinline__ void zero_slice(unsigned long long *const (&zero)[2], long long count, int part, int parts) {
+    if (!zero[0]) return;
+    const long long pairs = count / 2, per = (pairs + parts - 1) / parts;
+    const long long first = per * part, last = min(first + per, pairs);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        ulonglong2 *z = reinterpret_cast<ulonglong2 *>(zero[k]);
+        for (long long i = first + threadIdx.x; i < last; i += blockDim.x) z[i] = make_ulonglong2(0, 0);
+        if (part == 0 && threadIdx.x == 0 && (count & 1)) zero[k][count - 1] = 0;
+    }
 }
 
 // Tiles per row of an entry: 31 (SHARED) or 16 unclamped block columns each.
@@ -297,7 +331,13 @@ __device__ __forceinline__ void scan_tile_g(const MatchArgs &a, int bx, int by_c
             int pos = pack_pos(0, row) + (xb - R - 3);
             float st[4];
             scan_step_append<M, SHARED, GF, true, 3, 3, 4>(pc, pp, g, nc, st, pos, base, end, e, q);
-            for (int m = 1; m < (R + 1) / 2; ++m) {
+            int m = 1;
+            for (; m + 1 < (R + 1) / 2; m += 2) {
+                scan_two_steps<M, SHARED, GF>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
+                pc += 8;
+                pos += 8;
+            }
+            if (m < (R + 1) / 2) {
                 pc += 4;
                 pos += 4;
                 scan_step_append<M, SHARED, GF, false, 3, 0, 4>(pc, pp, g, nc, st, pos, base, end, e, q);

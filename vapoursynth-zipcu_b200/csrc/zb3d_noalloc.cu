@@ -128,9 +128,7 @@ extern "C" int zb3d_bm3d_plane_noalloc(const float *d_src, float *d_dst, int wid
     unsigned long long *den = reinterpret_cast<unsigned long long *>(base + kAccBytes);
     int2 *list = reinterpret_cast<int2 *>(base + 2 * kAccBytes);
 
-    // the array keeps the previous call's sums: both accumulators start from zero
-    cudaError_t e = cudaMemsetAsync(num, 0, pixels * sizeof(unsigned long long), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(den, 0, pixels * sizeof(unsigned long long), st);
+    cudaError_t e = cudaSuccess;
 
     // scaled sigma as the reference host stores it (vszipcu src/bm3d.zig:1019-1024)
     const unsigned bits = final_ ? 0x3e40c0c1u : 0x3f021bb6u;
@@ -150,6 +148,10 @@ extern "C" int zb3d_bm3d_plane_noalloc(const float *d_src, float *d_dst, int wid
     ma.nby = nby;
     ma.nbx_al = (width - 8) / block_step + 1;
     ma.list = list;
+    // the array keeps the previous call's sums: both accumulators start from zero
+    ma.zero[0] = num;
+    ma.zero[1] = den;
+    ma.zero_count = (long long)pixels;
     bool tiled = block_step == 4 || block_step == 8;
     if (tiled) {
         MatchArgs t = ma;
