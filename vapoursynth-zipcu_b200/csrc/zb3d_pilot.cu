@@ -11,13 +11,21 @@
 // weights [cout][ky][kx][cin], i.e. each output channel's 9 * cin inputs are
 // contiguous (the GEMM's K order); biases and gradients FP32.
 //
-// Forward: implicit GEMM per 8 x 16-pixel tile (M = 128 pixels, N = cout,
+// Forward: implicit GEMM per 16 x 16-pixel tile (M = 256 pixels, N = cout,
 // K = 9 * cin) from a shared-memory halo tile and the layer's weights.  The
 // same kernel does the backward pass to the input with the weights flipped in
 // space and transposed in channels, and applies the ReLU derivative (the next
 // layer's forward activation > 0) in its epilogue.  The weight gradient is a
 // persistent kernel: GEMM with M = cout, N = cin per kernel tap, K = pixels,
 // one warp per tap, FP32 partials flushed once per CTA.
+//
+// What bounds them at the recipe's 32 crops of 64 x 64 (every layer stays in L2): the wait for a
+// tile's loads, so these are 16-byte cp.async copies, all of a CTA's in flight at once
+// (forward: one wave of 512 CTAs) or a tile ahead of the arithmetic (weight gradient),
+// and fragments come by ldmatrix (transposed for the gradient, whose K is the pixels).
+// 32 -> 32 channels, against 4-byte copies and elements one by one:
+// forward 29 -> 15 us, input gradient 33 -> 17 us, weight gradient 45 -> 26 us; one batch's gradients
+// 723 -> 477 us, where the launches from Python begin to show.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -26,9 +34,9 @@
 namespace zb {
 namespace pilot {
 
-constexpr int TW = 16, TH = 8;            // output tile: 16 columns x 8 rows = 128 pixels
-constexpr int HW = TW + 2, HH = TH + 2;   // halo tile
-constexpr int HPIX = HW * HH;
+constexpr int TW = 16, HW = TW + 2;       // tile columns, without and with the halo
+constexpr int FTH = 16, FHPIX = HW * (FTH + 2);  // forward: rows, halo pixels
+constexpr int GTH = 8, GHPIX = HW * (GTH + 2);   // weight gradient
 
 struct ConvArgs {
     const __nv_bfloat16 *x;   // [n][h][w][cin]
@@ -64,37 +72,71 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
+}
+
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
+}
+
+// 8 channels (16 bytes) global -> shared, zeros where !ok.  VEC: one asynchronous copy, for
+// buffers that start on 16 bytes; else element by element.
+template <bool VEC>
+__device__ __forceinline__ void copy8(__nv_bfloat16 *d, const __nv_bfloat16 *s, bool ok) {
+    if constexpr (VEC) {
+        const unsigned a = (unsigned)__cvta_generic_to_shared(d);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(a), "l"(s), "r"(ok ? 16 : 0) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d[i] = ok ? s[i] : __float2bfloat16_rn(0.0f);
+    }
+}
+
+// The pixels [y0, y0 + rows) x [x0, x0 + cols) of an NHWC image, C channels, zeros outside it.
+template <int C, int PP, int COLS, int PIX, int THREADS, bool VEC>
+__device__ __forceinline__ void stage_pixels(__nv_bfloat16 *d, const __nv_bfloat16 *img, int y0, int x0, int h, int w) {
+    constexpr int CH = C / 8;
+    for (int i = threadIdx.x; i < PIX * CH; i += THREADS) {
+        const int pix = i / CH, c = i - pix * CH;
+        const int yy = y0 + pix / COLS, xx = x0 + pix % COLS;
+        const bool ok = yy >= 0 && yy < h && xx >= 0 && xx < w;
+        copy8<VEC>(d + pix * PP + 8 * c, ok ? img + ((size_t)yy * w + xx) * C + 8 * c : img, ok);
+    }
+}
+
 template <int CIN, int COUT>
 struct FwdShape {
-    static constexpr int PP = CIN + 8;         // halo pixel pitch (bf16): conflict-free fragment loads
+    static constexpr int PP = CIN + 8;         // halo pixel pitch (bf16): conflict-free ldmatrix rows
     static constexpr int K = 9 * CIN;
     static constexpr int KP = K + 8;           // weight row pitch (bf16)
-    static constexpr int SMEM = (HPIX * PP + COUT * KP) * 2;
+    static constexpr int SMEM = (FHPIX * PP + COUT * KP) * 2;
 };
 
-// y = conv3x3(x) (+ bias, ReLU, mask); grid (ceil(w/16), ceil(h/8), n), 128 threads.
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) conv3x3(ConvArgs p) {
+// y = conv3x3(x) (+ bias, ReLU, mask); grid (ceil(w/16), ceil(h/16), n), 256 threads.
+template <int CIN, int COUT, bool VEC>
+__global__ void __launch_bounds__(256) conv3x3(ConvArgs p) {
     using S = FwdShape<CIN, COUT>;
     constexpr int NT = COUT / 8;
     extern __shared__ __align__(16) __nv_bfloat16 sm[];
     __nv_bfloat16 *sx = sm;
-    __nv_bfloat16 *sw = sm + HPIX * S::PP;
+    __nv_bfloat16 *sw = sm + FHPIX * S::PP;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH, img = blockIdx.z;
-    const __nv_bfloat16 *xin = p.x + (size_t)img * p.h * p.w * CIN;
-    for (int i = tid; i < HPIX * (CIN / 2); i += 128) {
-        const int pix = i / (CIN / 2), cp = i - pix * (CIN / 2);
-        const int yy = y0 - 1 + pix / HW, xx = x0 - 1 + pix % HW;
-        uint32_t v = 0;
-        if (yy >= 0 && yy < p.h && xx >= 0 && xx < p.w)
-            v = reinterpret_cast<const uint32_t *>(xin + ((size_t)yy * p.w + xx) * CIN)[cp];
-        reinterpret_cast<uint32_t *>(sx + pix * S::PP)[cp] = v;
+    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * FTH, img = blockIdx.z;
+    stage_pixels<CIN, S::PP, HW, FHPIX, 256, VEC>(sx, p.x + (size_t)img * p.h * p.w * CIN, y0 - 1, x0 - 1, p.h, p.w);
+    for (int i = tid; i < COUT * (S::K / 8); i += 256) {
+        const int co = i / (S::K / 8), kc = i - co * (S::K / 8);
+        copy8<VEC>(sw + co * S::KP + 8 * kc, p.wgt + (size_t)co * S::K + 8 * kc, true);
     }
-    for (int i = tid; i < COUT * (S::K / 2); i += 128) {
-        const int co = i / (S::K / 2), kp = i - co * (S::K / 2);
-        reinterpret_cast<uint32_t *>(sw + co * S::KP)[kp] = reinterpret_cast<const uint32_t *>(p.wgt + (size_t)co * S::K)[kp];
-    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
 
     float acc[2][NT][4];
@@ -105,6 +147,8 @@ __global__ void __launch_bounds__(128) conv3x3(ConvArgs p) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[mt][nt][k] = 0.0f;
     // warp w: output rows 2w and 2w + 1 (one m16 tile each: pixels = the row's 16 columns)
+    const __nv_bfloat16 *arow = sx + (2 * warp * HW + (lane & 15)) * S::PP + 8 * (lane >> 4);
+    const __nv_bfloat16 *brow = sw + ((lane & 7) + ((lane >> 4) << 3)) * S::KP + 8 * ((lane >> 3) & 1);
 #pragma unroll 1
     for (int tap = 0; tap < 9; ++tap) {
         const int ky = tap / 3, kx = tap - 3 * ky;
@@ -112,19 +156,16 @@ __global__ void __launch_bounds__(128) conv3x3(ConvArgs p) {
         for (int cc = 0; cc < CIN; cc += 16) {
             uint32_t a[2][4];
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                const __nv_bfloat16 *base = sx + ((2 * warp + mt + ky) * HW + kx) * S::PP + cc + 2 * tig;
-                a[mt][0] = ld32(base + g * S::PP);
-                a[mt][1] = ld32(base + (g + 8) * S::PP);
-                a[mt][2] = ld32(base + g * S::PP + 8);
-                a[mt][3] = ld32(base + (g + 8) * S::PP + 8);
-            }
+            for (int mt = 0; mt < 2; ++mt) ldsm4(a[mt], arow + ((mt + ky) * HW + kx) * S::PP + cc);
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                const __nv_bfloat16 *wb = sw + (nt * 8 + g) * S::KP + tap * CIN + cc + 2 * tig;
-                const uint32_t b[2] = {ld32(wb), ld32(wb + 8)};
-                mma_bf16(acc[0][nt], a[0], b);
-                mma_bf16(acc[1][nt], a[1], b);
+            for (int nt = 0; nt < NT; nt += 2) {
+                uint32_t b[4];  // output channels 8 nt .. 8 nt + 15
+                ldsm4(b, brow + nt * 8 * S::KP + tap * CIN + cc);
+                const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+                mma_bf16(acc[0][nt], a[0], b0);
+                mma_bf16(acc[1][nt], a[1], b0);
+                mma_bf16(acc[0][nt + 1], a[0], b1);
+                mma_bf16(acc[1][nt + 1], a[1], b1);
             }
         }
     }
@@ -167,78 +208,80 @@ __global__ void __launch_bounds__(128) conv3x3(ConvArgs p) {
 
 template <int CIN, int COUT>
 struct WgShape {
-    static constexpr int DP = TW * TH + 8;     // transposed gradient tile pitch (pixels)
-    static constexpr int XP = HPIX + 6;        // transposed halo pitch (pixels)
-    static constexpr int SMEM = (COUT * DP + CIN * XP) * 2;
+    static constexpr int DP = COUT + 8, XP = CIN + 8;  // pixel pitches (bf16): conflict-free ldmatrix rows
+    static constexpr int DY = TW * GTH * DP, BUF = DY + GHPIX * XP;
+    static constexpr int SMEM = 2 * BUF * 2;           // two tiles
 };
 
 // dw[co][tap][ci] += sum over pixels dy[p][co] * x[p + tap offset][ci]; db[co] += sum dy[p][co].
-// Persistent: CTA b handles tiles b, b + gridDim.x, ...; 9 warps (one per tap) + the bias sums.
-template <int CIN, int COUT>
+// Persistent: CTA b handles tiles b, b + gridDim.x, ..., staging the next one while it computes;
+// 9 warps, one per tap, and the middle one multiplies by ones for the bias.
+template <int CIN, int COUT, bool VEC>
 __global__ void __launch_bounds__(288) conv3x3_wgrad(WgradArgs p) {
     using S = WgShape<CIN, COUT>;
     constexpr int MT = COUT / 16, NT = CIN / 8;
     extern __shared__ __align__(16) __nv_bfloat16 sm[];
-    __nv_bfloat16 *dyT = sm;                    // [COUT][DP]: pixel index r * 16 + c
-    __nv_bfloat16 *xT = sm + COUT * S::DP;      // [CIN][XP]:  halo index hr * 18 + hc
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int ky = warp / 3, kx = warp - 3 * ky;
-    const int tx = (p.w + TW - 1) / TW, ty = (p.h + TH - 1) / TH;
+    const int tx = (p.w + TW - 1) / TW, ty = (p.h + GTH - 1) / GTH;
     const long long ntiles = (long long)tx * ty * p.n;
-    float acc[MT][NT][4];
+    float acc[MT][NT][4], bacc[MT][4];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[mt][nt][k] = 0.0f;
-    float bsum = 0.0f;  // thread tid < COUT: bias gradient of channel tid
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) bacc[mt][k] = 0.0f;
+    }
+    auto stage = [&](long long t, __nv_bfloat16 *buf) {
         const int img = (int)(t / ((long long)tx * ty));
         const int rem = (int)(t - (long long)img * tx * ty);
-        const int y0 = (rem / tx) * TH, x0 = (rem % tx) * TW;
+        const int y0 = (rem / tx) * GTH, x0 = (rem % tx) * TW;
         const size_t base = (size_t)img * p.h * p.w;
-        __syncthreads();  // the previous tile's fragments are consumed
-        for (int i = tid; i < TW * TH * COUT; i += 288) {
-            const int pix = i / COUT, co = i - pix * COUT;
-            const int yy = y0 + pix / TW, xx = x0 + pix % TW;
-            __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
-            if (yy < p.h && xx < p.w) v = p.dy[(base + (size_t)yy * p.w + xx) * COUT + co];
-            dyT[co * S::DP + pix] = v;
-        }
-        for (int i = tid; i < HPIX * CIN; i += 288) {
-            const int hp = i / CIN, ci = i - hp * CIN;
-            const int yy = y0 - 1 + hp / HW, xx = x0 - 1 + hp % HW;
-            __nv_bfloat16 v = __float2bfloat16_rn(0.0f);
-            if (yy >= 0 && yy < p.h && xx >= 0 && xx < p.w) v = p.x[(base + (size_t)yy * p.w + xx) * CIN + ci];
-            xT[ci * S::XP + hp] = v;
+        stage_pixels<COUT, S::DP, TW, TW * GTH, 288, VEC>(buf, p.dy + base * COUT, y0, x0, p.h, p.w);
+        stage_pixels<CIN, S::XP, HW, GHPIX, 288, VEC>(buf + S::DY, p.x + base * CIN, y0 - 1, x0 - 1, p.h, p.w);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // ldmatrix rows are pixels (K), transposed on the way: lane -> (K row, first channel)
+    const int arow = (lane & 7) + ((lane >> 4) << 3), ach = 8 * ((lane >> 3) & 1);
+    const int brow = lane & 15, bch = 8 * (lane >> 4);
+    const uint32_t one2 = 0x3f803f80u, ones[2] = {one2, one2};  // bf16 1.0
+    int cur = 0;
+    if (blockIdx.x < ntiles) stage(blockIdx.x, sm);
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, cur ^= 1) {
+        const long long next = t + gridDim.x;
+        if (next < ntiles) {
+            stage(next, sm + (cur ^ 1) * S::BUF);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         }
         __syncthreads();
-        if (tid < COUT) {
-            float s = 0.0f;
-            for (int q = 0; q < TW * TH; ++q) s += __bfloat162float(dyT[tid * S::DP + q]);
-            bsum += s;
-        }
+        const __nv_bfloat16 *dy = sm + cur * S::BUF, *x = dy + S::DY;
 #pragma unroll 1
-        for (int r = 0; r < TH; ++r) {  // K step = the 16 pixels of tile row r
+        for (int r = 0; r < GTH; ++r) {  // K step = the 16 pixels of tile row r
             uint32_t a[MT][4];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                const __nv_bfloat16 *d = dyT + (16 * mt + g) * S::DP + 16 * r + 2 * tig;
-                a[mt][0] = ld32(d);
-                a[mt][1] = ld32(d + 8 * S::DP);
-                a[mt][2] = ld32(d + 8);
-                a[mt][3] = ld32(d + 8 * S::DP + 8);
-            }
-            const int h0 = (r + ky) * HW + kx + 2 * tig;  // halo index of pixel column 2 tig
+            for (int mt = 0; mt < MT; ++mt) ldsm4_t(a[mt], dy + (16 * r + arow) * S::DP + 16 * mt + ach);
+            const __nv_bfloat16 *xr = x + ((r + ky) * HW + kx + brow) * S::XP + bch;
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                const __nv_bfloat16 *xs = xT + (8 * nt + g) * S::XP + h0;
-                const uint32_t b[2] = {pack2(xs[0], xs[1]), pack2(xs[8], xs[9])};
+            for (int nt = 0; nt < NT; nt += 2) {
+                uint32_t b[4];  // input channels 8 nt .. 8 nt + 15
+                ldsm4_t(b, xr + 8 * nt);
+                const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) mma_bf16(acc[mt][nt], a[mt], b);
+                for (int mt = 0; mt < MT; ++mt) {
+                    mma_bf16(acc[mt][nt], a[mt], b0);
+                    mma_bf16(acc[mt][nt + 1], a[mt], b1);
+                }
             }
+            if (warp == 4)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) mma_bf16(bacc[mt], a[mt], ones);
         }
+        __syncthreads();  // the tile's fragments are consumed
     }
     // flush: c0, c1 -> co = 16 mt + g, ci = 8 nt + 2 tig (+1); c2, c3 -> co + 8
     const int tap = warp;
@@ -254,7 +297,12 @@ __global__ void __launch_bounds__(288) conv3x3_wgrad(WgradArgs p) {
             atomicAdd(d1, acc[mt][nt][2]);
             atomicAdd(d1 + 1, acc[mt][nt][3]);
         }
-    if (tid < COUT && p.db) atomicAdd(p.db + tid, bsum);
+    if (warp == 4 && tig == 0 && p.db)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {  // every column of the product with ones is the sum
+            atomicAdd(p.db + 16 * mt + g, bacc[mt][0]);
+            atomicAdd(p.db + 16 * mt + g + 8, bacc[mt][2]);
+        }
 }
 
 // ---- element-wise kernels ------------------------------------------------------
@@ -329,27 +377,30 @@ __global__ void f32_to_bf16(const float *a, long long count, __nv_bfloat16 *b) {
 
 // ---- launchers -----------------------------------------------------------------------
 
+static bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
+
 template <int CIN, int COUT>
 static cudaError_t conv_t(const pilot::ConvArgs &a, cudaStream_t st) {
     using S = pilot::FwdShape<CIN, COUT>;
-    auto k = pilot::conv3x3<CIN, COUT>;
+    auto k = aligned16(a.x) && aligned16(a.wgt) ? pilot::conv3x3<CIN, COUT, true> : pilot::conv3x3<CIN, COUT, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) return e;
-    const dim3 grid((a.w + pilot::TW - 1) / pilot::TW, (a.h + pilot::TH - 1) / pilot::TH, a.n);
-    k<<<grid, 128, S::SMEM, st>>>(a);
+    const dim3 grid((a.w + pilot::TW - 1) / pilot::TW, (a.h + pilot::FTH - 1) / pilot::FTH, a.n);
+    k<<<grid, 256, S::SMEM, st>>>(a);
     return cudaGetLastError();
 }
 
 template <int CIN, int COUT>
 static cudaError_t wgrad_t(const pilot::WgradArgs &a, cudaStream_t st) {
     using S = pilot::WgShape<CIN, COUT>;
-    auto k = pilot::conv3x3_wgrad<CIN, COUT>;
+    auto k = aligned16(a.x) && aligned16(a.dy) ? pilot::conv3x3_wgrad<CIN, COUT, true>
+                                               : pilot::conv3x3_wgrad<CIN, COUT, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long tiles = (long long)((a.w + pilot::TW - 1) / pilot::TW) * ((a.h + pilot::TH - 1) / pilot::TH) * a.n;
+    const long long tiles = (long long)((a.w + pilot::TW - 1) / pilot::TW) * ((a.h + pilot::GTH - 1) / pilot::GTH) * a.n;
     const int grid = (int)(tiles < 2LL * sms ? tiles : 2LL * sms);
     k<<<grid, 288, S::SMEM, st>>>(a);
     return cudaGetLastError();
