@@ -1,8 +1,7 @@
 """The row kernel of the temporal search (ssd, ps_num 1 and 2, ps_range 2 to 6): its lists equal the
 CPU oracle's for every window size, at planes smaller than a window and with windows cut by the
 plane's edges, with content full of ties, with infinities and NaN, and with a number of blocks
-that leaves the last warp's groups idle.  A source that does not start on 16 bytes takes the
-other kernel and gives the same lists.
+that leaves the last warp's groups idle.  A source that does not start on 16 bytes gives the same lists.
 """
 import numpy as np
 import pytest

@@ -12,12 +12,15 @@
 // reads for ps_num <= 2).
 //
 // What bounds it: the FMA pipe (576 packed operations per lane and window; 27 of 32 lanes have
-// a row) and the wait for a window's loads, whose place the window before decides.  The
-// lane-pair form that it replaces (zb_match_temporal, still used for other metrics, ps_num > 2,
-// other window sizes and unaligned planes) read its windows through L1 with one lane pair per
-// block and waited on those loads: 1920x1080, block_step 8, radius 2 (21.0 M candidates): 355 ->
-// about 190 us; ps_range 2 124 -> 110, 6 670 -> 370.  With 168 registers (3 CTAs per SM) 6%
-// slower; with the window's loads in two halves (no spill) 10% slower.
+// a row), shared with the load-store unit's 128 column reads and 32 copies per window.  A
+// window's place is only known once an earlier one is done, so the two directions take turns
+// and the next window is copied (cp.async, a second buffer) while this one is scanned.
+// 1920x1080, block_step 8, radius 2 (21.0 M candidates): 355 us for the lane-pair form that this
+// replaces (zb_match_temporal, still used for other metrics, ps_num > 2 and other window sizes:
+// it reads its windows through L1 with one lane pair per block and waits on those loads), about
+// 190 us here; ps_range 2 124 -> 95, 3 218 -> 133, 5 490 -> 340, 6 670 -> 395.  Windows loaded to
+// registers ahead of each scan instead of copied under it: the same alone, 2.5% slower a
+// window among others, and only for 16-byte aligned planes.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -34,11 +37,12 @@ struct TempShape {
     static constexpr int G = 2 * P + 1;              // lanes per group, candidate rows and columns of a window
     static constexpr int NG = 32 / G;                // groups per warp
     static constexpr int N = 2 * P + 8;              // window side in pixels
-    static constexpr int CH = (N + 3 + 3) / 4;       // 16-byte chunks per staged row
+    static constexpr int LN = G < 8 ? G : 8;         // lanes that copy a row
     static constexpr int PITCH = N | 1;              // floats per row: odd
     // floats between the groups' windows; for P = 4 the rows of the three groups (at 0, 10 and 20
     // mod 32, 17 floats apart) are on 27 different banks
     static constexpr int WIN = N * PITCH + 26;
+    static constexpr int BUF = NG * WIN;             // floats of a warp's windows; each warp has two sets
 };
 
 // Strict-less insertion into a list of two.
@@ -50,61 +54,43 @@ __device__ __forceinline__ void top2_insert(float &e0, int &q0, float &e1, int &
     e0 = fminf(e0, err);
 }
 
-// The group's window of frame plane fp around (xx, yy): the first two candidates in scan
-// order, on every lane of the group.  r: the lane's candidate row (>= G: a lane without one).
+// Starts the copy of the group's window of frame plane fp around (xx, yy) into win: LN lanes on
+// LN consecutive pixels, row after row.  Rows and columns past the plane are only read by
+// candidates that do not exist: clamped.
 template <int P>
-__device__ __forceinline__ void scan_window_group(const MatchArgs &a, const float *__restrict__ fp, int xx, int yy,
-                                                  int r, int lane, unsigned gmask, float *win, const float2 (&nc)[4][8], float &e0,
-                                                  int &q0, float &e1, int &q1) {
+__device__ __forceinline__ void stage_window_group(const MatchArgs &a, const float *__restrict__ fp, int xx, int yy,
+                                                   int r, float *win) {
     using S = TempShape<P>;
-    constexpr int G = S::G, N = S::N, CH = S::CH, PITCH = S::PITCH;
+    constexpr int N = S::N, LN = S::LN, CH = (N + LN - 1) / LN;
+    const int left = max(xx - P, 0), top = max(yy - P, 0);
+    if (r < LN) {
+        const int ymax = a.h - 1 - top;
+        const float *src[CH];
+#pragma unroll
+        for (int c = 0; c < CH; ++c) src[c] = fp + (long long)top * a.pitch + min(left + r + LN * c, a.w - 1);
+#pragma unroll
+        for (int row = 0; row < N; ++row) {
+            const long long o = (long long)min(row, ymax) * a.pitch;
+#pragma unroll
+            for (int c = 0; c < CH; ++c)
+                if (LN * (c + 1) <= N || r + LN * c < N)
+                    cp_async_f32(win + row * S::PITCH + r + LN * c, src[c] + o, true);
+        }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// The staged window around (xx, yy): its first two candidates in scan order, on every lane of
+// the group.  r: the lane's candidate row (>= G: a lane without one).
+template <int P>
+__device__ __forceinline__ void scan_window_group(const MatchArgs &a, int xx, int yy, int r, int lane, unsigned gmask,
+                                                  const float *win, const float2 (&nc)[4][8], float &e0, int &q0,
+                                                  float &e1, int &q1) {
+    using S = TempShape<P>;
+    constexpr int G = S::G, N = S::N, PITCH = S::PITCH;
     const int W = a.w, H = a.h;
     const int left = max(xx - P, 0), right = min(xx + P, W - 8);
     const int top = max(yy - P, 0), bottom = min(yy + P, H - 8);
-    const int off = left & 3, xa = left - off;
-    __syncwarp();  // the group has read its last window
-    {
-        // Rows and columns past the plane are only read by candidates that do not exist: clamped.
-        // Chunks 0..3 of RL rows per step (4 lanes on a row's 64 bytes), then the rest.
-        const int ymax = H - 1 - top;
-        const float *rows = fp + (long long)top * a.pitch;
-        constexpr int RL = G / 4, STEPS = (N + RL - 1) / RL;
-        const int u = r & 3, rl = r >> 2, c0 = 4 * u - off;
-        const float *src = rows + min(xa + 4 * u, a.pitch - 4);
-        if (rl < RL) {
-            float4 v[STEPS];  // all loads in flight before the first store
-#pragma unroll
-            for (int k = 0; k < STEPS; ++k)
-                v[k] = __ldg(reinterpret_cast<const float4 *>(src + (long long)min(RL * k + rl, ymax) * a.pitch));
-            float *d = win + rl * PITCH + c0;
-#pragma unroll
-            for (int k = 0; k < STEPS; ++k, d += RL * PITCH) {
-                if (RL * k + rl >= N) break;
-                if (c0 >= 0) d[0] = v[k].x;  // c0 <= N: at most the padding column
-                if (c0 + 1 >= 0 && c0 + 1 < N) d[1] = v[k].y;
-                if (c0 + 2 >= 0 && c0 + 2 < N) d[2] = v[k].z;
-                if (c0 + 3 < N) d[3] = v[k].w;
-            }
-        }
-        constexpr int EX = CH - 4;
-        if constexpr (EX > 0) {
-#pragma unroll
-            for (int k = 0; k < (N * EX + G - 1) / G; ++k) {
-                const int i = r + G * k, row = i / EX, uu = 4 + i - row * EX;
-                const int cc = 4 * uu - off;
-                if (r >= G || i >= N * EX || cc >= N) continue;
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(
-                    rows + (long long)min(row, ymax) * a.pitch + min(xa + 4 * uu, a.pitch - 4)));
-                float *d = win + row * PITCH + cc;
-                d[0] = v.x;
-                if (cc + 1 < N) d[1] = v.y;
-                if (cc + 2 < N) d[2] = v.z;
-                if (cc + 3 < N) d[3] = v.w;
-            }
-        }
-    }
-    __syncwarp();
-
     const int dy = min(r, G - 1);
     const bool rowok = r < G && top + dy <= bottom;
     const int nx = rowok ? right - left + 1 : 0;
@@ -173,7 +159,7 @@ template <int P>
 __global__ void __launch_bounds__(kTempWarps * 32, 4) zb_match_temporal_rows(MatchArgs a) {
     using S = TempShape<P>;
     constexpr int G = S::G, NG = S::NG;
-    __shared__ float wins[kTempWarps * NG * S::WIN];
+    __shared__ float wins[kTempWarps * 2 * S::BUF];
     extern __shared__ int2 found[];  // [group][direction][t][2]: the frame lists (error, position)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool member = lane < NG * G;
@@ -185,7 +171,7 @@ __global__ void __launch_bounds__(kTempWarps * 32, 4) zb_match_temporal_rows(Mat
     const int by = (int)(bi / a.nbx), kx = (int)(bi - (long long)by * a.nbx);
     const int W = a.w, H = a.h, R = a.radius;
     const int x = min(a.bs * kx, W - 8), y = min(a.bs * by, H - 8);
-    float *win = wins + (warp * NG + g) * S::WIN;
+    float *win = wins + warp * 2 * S::BUF + g * S::WIN;
     int2 *mine = found + (size_t)(warp * NG + g) * 4 * R;
 
     // the negated reference patch as row pairs (2k, 2k + 1) of its 8 columns
@@ -199,33 +185,53 @@ __global__ void __launch_bounds__(kTempWarps * 32, 4) zb_match_temporal_rows(Mat
                 nc[k][j] = make_float2(-__ldg(c + 2 * k * a.pitch + j), -__ldg(c + (2 * k + 1) * a.pitch + j));
     }
     const int2 l0 = a.list[bi * 8], l1 = a.list[bi * 8 + 1];
+    // Windows in the order t = 1..r, direction, i: the window after the current one is then
+    // always known (its centre comes from the same direction's frame t - 1), so it is copied
+    // while the current one is scanned.  Each direction starts from the spatial list.
+    const int s0 = pack_pos(l0.x, l0.y & 0xffffff), s1 = pack_pos(l1.x, l1.y & 0xffffff);
+    int p0 = s0, p1 = s1, o0 = s0, o1 = s1;  // centres: this direction's, the other's
+    float e0 = ZB_FLT_MAX, e1 = ZB_FLT_MAX, w0 = 0.0f, w1 = 0.0f;
+    int q0 = 0, q1 = 0, u0 = 0, u1 = 0;
+    const int per_frame = a.ps_num, items = 2 * R * per_frame;
+    auto frame_of = [&](int k) {  // plane of item k
+        const int f = k / per_frame, t = f / 2 + 1;
+        return a.frames + (long long)((f & 1) ? R + t : R - t) * a.fstride;
+    };
+    stage_window_group<P>(a, frame_of(0), pos_x(p0), pos_y(p0), r, win);
 #pragma unroll 1
-    for (int way = 0; way < 2; ++way) {
-        // each direction starts from the spatial list
-        int p0 = pack_pos(l0.x, l0.y & 0xffffff), p1 = pack_pos(l1.x, l1.y & 0xffffff);
-#pragma unroll 1
-        for (int t = 1; t <= R; ++t) {
-            const float *fp = a.frames + (long long)(way ? R + t : R - t) * a.fstride;
-            float e0 = ZB_FLT_MAX, e1 = ZB_FLT_MAX;
-            int q0 = 0, q1 = 0;
-            float w0, w1;
-            int u0, u1;
-#pragma unroll 1
-            for (int i = 0; i < a.ps_num; ++i) {
-                const int p = i ? p1 : p0;
-                // a second window at the same place has the same candidates
-                if (i == 0 || !__all_sync(kFull, p1 == p0))
-                    scan_window_group<P>(a, fp, pos_x(p), pos_y(p), r, lane, gmask, win, nc, w0, u0, w1, u1);
-                top2_insert(e0, q0, e1, q1, w0, u0);
-                top2_insert(e0, q0, e1, q1, w1, u1);
-            }
+    for (int k = 0; k < items; ++k) {
+        const int i = k - k / per_frame * per_frame;
+        const bool last = i == per_frame - 1;  // of its frame: the next item is the other direction's
+        float *cur = win + (k & 1) * S::BUF, *nxt = win + ((k + 1) & 1) * S::BUF;
+        if (k + 1 < items) {
+            const int c = last ? o0 : p1;
+            __syncwarp();  // the buffer's window has been read
+            stage_window_group<P>(a, frame_of(k + 1), pos_x(c), pos_y(c), r, nxt);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncwarp();
+        const int p = i ? p1 : p0;
+        // a second window at the same place has the same candidates
+        if (i == 0 || !__all_sync(kFull, p1 == p0))
+            scan_window_group<P>(a, pos_x(p), pos_y(p), r, lane, gmask, cur, nc, w0, u0, w1, u1);
+        top2_insert(e0, q0, e1, q1, w0, u0);
+        top2_insert(e0, q0, e1, q1, w1, u1);
+        if (last) {
+            const int f = k / per_frame;
             if (r == 0) {
-                int2 *o = mine + (way * R + t - 1) * 2;
+                int2 *o = mine + ((f & 1) * R + f / 2) * 2;
                 o[0] = make_int2(__float_as_int(e0), q0);
                 o[1] = make_int2(__float_as_int(e1), q1);
             }
-            p0 = q0;
-            p1 = q1;
+            // the other direction next; this one goes on from the frame's list
+            p0 = o0;
+            p1 = o1;
+            o0 = q0;
+            o1 = q1;
+            e0 = e1 = ZB_FLT_MAX;
+            q0 = q1 = 0;
         }
     }
     if (r != 0 || slot >= nb) return;
@@ -275,11 +281,9 @@ static cudaError_t launch_rows_t(const MatchArgs &a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Whether the row kernel takes this search: window rows that fill a warp well, and planes that
-// 16-byte loads can read (a caller's buffer may start anywhere).
+// Whether the row kernel takes this search: window rows that fill a warp well.
 bool temporal_rows_eligible(const MatchArgs &a, int metric) {
-    return metric == M_SSD && a.ps_num <= 2 && a.ps_range >= 2 && a.ps_range <= 6 &&
-           reinterpret_cast<uintptr_t>(a.frames) % 16 == 0 && a.pitch % 4 == 0 && a.fstride % 4 == 0;
+    return metric == M_SSD && a.ps_num >= 1 && a.ps_num <= 2 && a.ps_range >= 2 && a.ps_range <= 6;
 }
 
 cudaError_t launch_temporal_rows(const MatchArgs &a, cudaStream_t st) {
