@@ -293,7 +293,7 @@ void zb3d_host_free(void *p);
  * One window (the zb3d_process_device layout: d_src, d_dst of that filter) of each job,
  * all on the filters' device, in one call: the plane entries of every job that use SSD
  * matching at block_step 4 or 8 (FP32 scan), radius 0 and the DCT in both dimensions are
- * matched and filtered by one persistent launch per filter step over a work list (match
+ * matched and filtered by two launches per filter step over a work list (match
  * tiles of every entry, then filter chunks, each chunk waiting, bounded, for its entry's
  * matching), then finished; any other entry runs on its own as in zb3d_process_device.
  * The call returns when the outputs are written (it synchronises `stream`).  Returns 0,
