@@ -342,20 +342,23 @@ __global__ void __launch_bounds__(kFinishWarps * 32) zb_finish(FinishArgs a, int
         const int y = y0 - 8 + k;
         prev[k] = y >= 0 ? finish_load(den + (long long)y * a.pitch, x, a.w, vec) : make_longlong2(0, 0);
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        sa += prev[k].x;
-        sb += prev[k].y;
-    }
-    const int yend = min(y0 + rows, a.h);
-    for (int yc = y0; yc < yend; yc += 8) {
-        longlong2 cur[8], n[8];
+    longlong2 cur[8], n[8];
+    auto load = [&](int yc) {  // weights and numerators of 8 rows
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int y = min(yc + k, a.h - 1);
             cur[k] = finish_load(den + (long long)y * a.pitch, x, a.w, vec);
             n[k] = out ? finish_load(num + (long long)y * a.pitch, x, a.w, vec) : make_longlong2(0, 0);
         }
+    };
+    load(y0);  // before the sums below wait for their loads
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        sa += prev[k].x;
+        sb += prev[k].y;
+    }
+    const int yend = min(y0 + rows, a.h);
+    for (int yc = y0;;) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int y = yc + k;
@@ -391,6 +394,8 @@ __global__ void __launch_bounds__(kFinishWarps * 32) zb_finish(FinishArgs a, int
                 }
             }
         }
+        if ((yc += 8) >= yend) break;
+        load(yc);
     }
 }
 
@@ -438,7 +443,7 @@ __global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps *
         zero_slice(m.zero, m.zero_count, local, E.match_items);
         if (bx == m.tiles_x) {  // the clamped last block column
             const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
-            if (cy < m.nby) column_block<M_SSD>(m, cy);
+            if (cy < m.nby) warp_block<M_SSD>(m, m.nbx - 1, cy);
         } else if (m.bs == 4) {
             scan_tile<M_SSD, true, 4>(m, bx, by, kBatchMatchRows, dyn);
         } else {

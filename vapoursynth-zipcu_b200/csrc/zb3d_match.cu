@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128) zb_match_tiled(MatchArgs a) {
 template <int M>
 __global__ void __launch_bounds__(128) zb_match_column(MatchArgs a) {
     const int by = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (by < a.nby) column_block<M>(a, by);  // whole warps
+    if (by < a.nby) warp_block<M>(a, a.nbx - 1, by);  // whole warps
 }
 
 // Spatial SSD / SAD matching at block_step 4 and 8 (scan_tile), `rows` block rows per CTA of 8
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a,
     zero_slice(a.zero, a.zero_count, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
     if ((int)blockIdx.x == a.tiles_x) {
         const int warp = threadIdx.x >> 5, by = blockIdx.y * rows + warp;
-        if (warp < rows && by < a.nby) column_block<M>(a, by);
+        if (warp < rows && by < a.nby) warp_block<M>(a, a.nbx - 1, by);
         return;
     }
     scan_tile<M, SHARED, BS>(a, blockIdx.x, blockIdx.y, rows, tile);
@@ -382,8 +382,28 @@ static cudaError_t launch_tiled_m(MatchArgs a, int rows_per_cta, cudaStream_t st
     return launch_tiled_t<M, false, 4>(a, rows_per_cta, st);
 }
 
+// Every block of a small plane, a warp per block.
+template <int M>
+__global__ void __launch_bounds__(128) zb_match_blocks(MatchArgs a) {
+    const int bi = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (bi >= a.nby * a.nbx) return;  // whole warps
+    const int by = bi / a.nbx;
+    warp_block<M>(a, bi - by * a.nbx, by);
+}
+
+// Up to this many blocks (one wave of 16 warps per SM) a warp takes a block; a lane pair per
+// block (zb_match_global) does a third of the work but leaves a plane of this size on at most
+// 148 warps: block_step 5,
+// bm_range 9, 320 blocks 105 -> 21 us, 960 blocks 105 -> 27 us.  Above it three streams fill the
+// GPU with lane pairs and the work counts.
+constexpr long long kWarpBlocks = 148 * 16;
+
 template <int M>
 static cudaError_t launch_global_m(const MatchArgs &a, cudaStream_t st) {
+    if (a.gen_mode == 0 && (long long)a.nby * a.nbx <= kWarpBlocks) {
+        zb_match_blocks<M><<<(unsigned)((a.nby * a.nbx + 3) / 4), 128, 0, st>>>(a);
+        return cudaGetLastError();
+    }
     // listed blocks (gen_mode 2): the count is on the device, so size for every block
     const long long threads = (long long)a.nby * a.nbx * 2;
     zb_match_global<M><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(a);

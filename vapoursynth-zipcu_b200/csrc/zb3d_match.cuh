@@ -358,17 +358,16 @@ __device__ __forceinline__ void neg_pairs(const float (&c)[8][4], float2 (&nc)[4
         for (int j = 0; j < 4; ++j) nc[k][j] = make_float2(-c[2 * k][j], -c[2 * k + 1][j]);
 }
 
-// The clamped last block column (x = W - 8) that the tiled kernels leave out: one warp per
-// block.  Its candidate rows are split into 16 consecutive ranges in order, one per lane
+// One block by a whole warp: the clamped last block column (x = W - 8) that the tiled kernels
+// leave out, and every block of small planes at the other block steps.  Its candidate rows are split into 16 consecutive ranges in order, one per lane
 // pair, each scanned in the reference's order into a list of its own; the lists are then
 // merged in row order, a later range's entries inserted (strict less) after the earlier
 // ranges', which is the list of one scan over all the rows.
 template <int M>
-__device__ __forceinline__ void column_block(const MatchArgs &a, int by) {
+__device__ __forceinline__ void warp_block(const MatchArgs &a, int kx, int by) {
     const int lane = threadIdx.x & 31;
     const int hh = lane & 1, pr = lane >> 1;
     const int W = a.w, H = a.h, R = a.range;
-    const int kx = a.nbx - 1;
     const int x = min(a.bs * kx, W - 8), y = min(a.bs * by, H - 8);
     const unsigned pm = 3u << (lane & 30);
     const float *plane = a.frames + (long long)a.radius * a.fstride + 4 * hh;
