@@ -284,6 +284,7 @@ __device__ __forceinline__ void filter8_groups(const FilterArgs &a, long long g0
     float *xb = gb + col_off(l8, 0), *xs = gb + col_off(l8, 1);  // layout X, the two row halves
     long long *off = offs + gi * kOffStride;
     const float E = a.extractor, E32 = E * kFixScale;
+    __syncwarp();  // a caller's previous groups: their offsets have been read
     {
         const int2 v = a.list[grp * 8 + l8];
         const long long z = (unsigned)v.y >> 24, yx = (long long)(v.y & 0xffffff) * a.pitch + v.x;
