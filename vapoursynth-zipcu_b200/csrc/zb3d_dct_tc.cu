@@ -126,7 +126,8 @@ __device__ __forceinline__ void tma_store_box(const CUtensorMap *map, int col, i
 }
 
 // Bounded wait on an mbarrier phase; gives up at once when another role has aborted.  On
-// timeout it sets the abort flag and status 1.
+// timeout it sets the abort flag and status 1.  Lanes can end it differently: a warp that
+// goes on to warp-wide operations votes on the result, so that it leaves together.
 __device__ __forceinline__ bool wait_phase(uint32_t mbar, uint32_t parity, volatile int *abort_flag, int *status) {
     for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
         if (mbar_try(mbar, parity)) return true;
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
 #pragma unroll
                 for (int y = 0; y < 8; ++y) d[q][y] = ok ? __ldg(p + (long long)y * src.pitch) : 0.0f;
             }
-            if (!wait_phase(sfree(s), (u & 1u) ^ 1u, abort_flag, status)) break;
+            if (!__all_sync(0xffffffffu, wait_phase(sfree(s), (u & 1u) ^ 1u, abort_flag, status))) break;
             uint8_t *hi = sm + s * STAGE_BYTES, *lo = hi + 2 * HALF_BYTES;
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
         for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, ++li) {
             const int s = (int)(li % STAGES);
             const uint32_t u = (uint32_t)(li / STAGES);
-            if (!wait_phase(full(s), u & 1u, abort_flag, status)) break;
+            if (!__all_sync(0xffffffffu, wait_phase(full(s), u & 1u, abort_flag, status))) break;
             float4 *hi = reinterpret_cast<float4 *>(sm + s * STAGE_BYTES);
             float4 *lo = reinterpret_cast<float4 *>(sm + s * STAGE_BYTES + 2 * HALF_BYTES);
 #pragma unroll 4
@@ -322,8 +323,7 @@ __global__ void __launch_bounds__(GATHER ? THREADS_GATHER : THREADS, 1)
         for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, ++li) {
             const int s = (int)(li % STAGES);
             const uint32_t u = (uint32_t)(li / STAGES);
-            const bool ok = wait_phase(accf(s), u & 1u, abort_flag, status);
-            if (!__all_sync(0xffffffffu, ok)) break;
+            if (!__all_sync(0xffffffffu, wait_phase(accf(s), u & 1u, abort_flag, status))) break;
             fence_after_sync();
             float v[32], w[32];
             const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(s * 64);

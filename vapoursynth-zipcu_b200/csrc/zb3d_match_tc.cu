@@ -654,7 +654,8 @@ __global__ void __launch_bounds__(THREADS, 1) zb_match_tc(MatchArgs a) {
             const bool pass2 = j >= nch;
             if (pass2 && !have_t) exchange();
             const long long tw0 = prof ? clock64() : 0;
-            if (!mbar_wait(done0 + 8 * s, (j >> 1) & 1, polls)) {
+            // a vote: the warp leaves together for the boundary below, or goes on together
+            if (!__all_sync(0xffffffffu, mbar_wait(done0 + 8 * s, (j >> 1) & 1, polls))) {
                 timeout = 1;
                 break;
             }

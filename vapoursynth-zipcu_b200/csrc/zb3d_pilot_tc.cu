@@ -127,7 +127,8 @@ __device__ __forceinline__ uint64_t desc_k(uint32_t saddr, uint32_t lbo, uint32_
 
 // Waits for phase `parity` of an mbarrier.  Gives up when another role has
 // aborted, or after WAIT_LIMIT tries: then it raises the abort flag and records
-// `code` in the status word.
+// `code` in the status word.  Lanes can end it differently: a warp that goes on to warp-wide
+// operations votes on the result, so that it leaves together.
 __device__ __forceinline__ bool wait_bar(uint32_t mbar, uint32_t parity, volatile int *abort_flag, int *status,
                                          int code) {
     for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(Shape<CIN, COUT>::THREADS, Shape<CIN, COUT>::C
             for (int j = 0; j < n + 4; ++j, ++g) {
                 if ((int)(g % S::EPI_GROUPS) != grp) continue;
                 const int slot = acc_slot(g);
-                if (!wait_bar(acc_full + 8u * slot, (g / NACC) & 1, abort_flag, p.status, 4)) {
+                if (!__all_sync(0xffffffffu, wait_bar(acc_full + 8u * slot, (g / NACC) & 1, abort_flag, p.status, 4))) {
                     ok = false;
                     break;
                 }
