@@ -1,6 +1,7 @@
 // zb3d_filter.cuh on the CPU (cuda_runtime.h beside this file stands in for CUDA).
 //   filter8 chunk <final> <descending>   one chunk of groups (the last 8 short of 3) in one set of buffers, as the batch
 //       kernel runs it, against the same groups 8 at a time in fresh buffers: equal sums or exit 1
+//   filter8 sums <final> <extractor exponent>   prints how many numerators and weights are not 0
 #include "cuda_runtime.h"
 #include "zb3d_filter.cuh"
 
@@ -14,7 +15,7 @@ struct Job {
     std::vector<unsigned long long> num, den;
     FilterArgs a{};
 
-    Job(int groups) : src(2 * PLANES * W * H), list(groups * 8), num(PLANES * W * H), den(PLANES * W * H) {
+    Job(int groups, float extractor) : src(2 * PLANES * W * H), list(groups * 8), num(PLANES * W * H), den(PLANES * W * H) {
         unsigned s = 12345;
         auto next = [&] { return (s = s * 1664525u + 1013904223u) >> 8; };
         for (float &v : src) v = next() * (1.0f / 16777216.0f);
@@ -29,7 +30,7 @@ struct Job {
         a.list = list.data();
         a.nblocks = groups;
         for (float &v : a.sigma) v = 0.4f;
-        a.extractor = 8.0f;
+        a.extractor = extractor;
         a.num = num.data();
         a.den = den.data();
     }
@@ -51,7 +52,7 @@ void run(const FilterArgs &a, Buffers &b, long long g0, long long g1, bool desce
 
 template <bool FINAL>
 int chunk(bool descending) {
-    Job one(GROUPS), eight(GROUPS);
+    Job one(GROUPS, 8.0f), eight(GROUPS, 8.0f);
     auto b = std::make_unique<Buffers>();
     run<FINAL>(one.a, *b, 0, GROUPS, descending);
     for (int g = 0; g < GROUPS; g += kFilterGroups) {
@@ -61,8 +62,21 @@ int chunk(bool descending) {
     return one.num == eight.num && one.den == eight.den ? 0 : 1;
 }
 
+template <bool FINAL>
+int sums(int exponent) {
+    Job j(kFilterGroups, std::ldexp(1.0f, exponent));
+    auto b = std::make_unique<Buffers>();
+    run<FINAL>(j.a, *b, 0, kFilterGroups, false);
+    int n = 0, d = 0;
+    for (unsigned long long v : j.num) n += v != 0;
+    for (unsigned long long v : j.den) d += v != 0;
+    printf("%d %d\n", n, d);
+    return 0;
+}
+
 int main(int argc, char **argv) {
-    if (argc != 4 || strcmp(argv[1], "chunk")) return 2;
-    const bool descending = atoi(argv[3]) != 0;
-    return atoi(argv[2]) ? chunk<true>(descending) : chunk<false>(descending);
+    if (argc != 4) return 2;
+    const int final_ = atoi(argv[2]), v = atoi(argv[3]);
+    if (!strcmp(argv[1], "chunk")) return final_ ? chunk<true>(v != 0) : chunk<false>(v != 0);
+    return final_ ? sums<true>(v) : sums<false>(v);
 }

@@ -22,3 +22,12 @@ def filter8(tmp_path_factory):
 @pytest.mark.parametrize("descending", [0, 1])
 def test_groups_after_groups_in_the_same_buffers(filter8, final, descending):
     assert subprocess.run([filter8, "chunk", str(final), str(descending)]).returncode == 0
+
+
+@pytest.mark.parametrize("final", [0, 1])
+@pytest.mark.parametrize("exponent,rounds_to_zero", [(3, False), (95, True), (96, True), (100, True), (127, True)])
+def test_extractor_exponents(filter8, final, exponent, rounds_to_zero):
+    """v + 2^e - 2^e: the spacing of floats at 2^e is 2^(e - 23), so with e from 26 up every weighted pixel and weight of [0, 1] data rounds to
+    zero, also where 2^e scaled to the accumulators' fixed point would be infinite."""
+    counts = list(map(int, subprocess.check_output([filter8, "sums", str(final), str(exponent)]).split()))
+    assert (counts == [0, 0]) == rounds_to_zero, counts

@@ -27,8 +27,9 @@
 // operation is stated, in the form that equals the compiler's on the reference's code shape,
 // found by comparing every form on random lines: the forward transform fuses everywhere; the
 // inverse joins its two even products (coefficients 0 and 4) in three ways, by what feeds it
-// (DctIn).  The 1/4096 of the unnormalised 3D pair is applied with the weight, and the
-// 2^32 of the fixed point before the extractor's rounding: a power of two commutes with both.
+// (DctIn).  The 1/4096 of the unnormalised 3D pair is applied with the weight: a power of two
+// commutes with the roundings before it.  The 2^32 of the fixed point comes after the extractor,
+// whose 2^e may be any float.
 #pragma once
 #include "zb3d_args.h"
 #include "zb3d_match.cuh"
@@ -283,7 +284,7 @@ __device__ __forceinline__ void filter8_groups(const FilterArgs &a, long long g0
     float *patch = gb + l8 * kPatchStride;                       // layout P
     float *xb = gb + col_off(l8, 0), *xs = gb + col_off(l8, 1);  // layout X, the two row halves
     long long *off = offs + gi * kOffStride;
-    const float E = a.extractor, E32 = E * kFixScale;
+    const float E = a.extractor;
     __syncwarp();  // a caller's previous groups: their offsets have been read
     {
         const int2 v = a.list[grp * 8 + l8];
@@ -360,7 +361,7 @@ __device__ __forceinline__ void filter8_groups(const FilterArgs &a, long long g0
         k += __shfl_xor_sync(kFull, k, 2);
         k += __shfl_xor_sync(kFull, k, 4);
         const float w = 1.0f / k;
-        const float ws = w * (kFixScale / 4096.0f);
+        const float ws = w * (1.0f / 4096.0f);
         __syncwarp();
         horizontal<true>(patch);
         __syncwarp();
@@ -375,7 +376,7 @@ __device__ __forceinline__ void filter8_groups(const FilterArgs &a, long long g0
             unsigned long long *q = num + off[8 + p];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                const float2 v = __fadd2_rn(__ffma2_rn(pk(ws), d[r][p], pk(E32)), pk(-E32));
+                const float2 v = pmul(kFixScale, __fadd2_rn(__ffma2_rn(pk(ws), d[r][p], pk(E)), pk(-E)));
                 atomicAdd(q, to_fix(v.x));
                 q += a.pitch;
                 atomicAdd(q, to_fix(v.y));
