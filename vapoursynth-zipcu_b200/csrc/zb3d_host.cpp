@@ -547,17 +547,20 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     if (f->match_form != 1 || !tc_ok) {
         if (tiled && !entry_scan_fits(e, 1))
             for (int r : {2, 4}) cands.push_back({0, r});
-        // from 8 rows down; a plane that already has 4 waves of CTAs (2 per SM) gains nothing
-        // from more of them, and a tile that leaves one CTA per SM is only taken for want of others
-        int last = 0;
-        for (int r = 8; r >= 1; r >>= 1) {
-            if (!entry_scan_fits(e, r)) continue;
-            if (last && !entry_scan_fits2(e, last)) cands.clear();
-            else if (last && scan_ctas(e, last) >= 8LL * sms) break;
+        // from 8 rows down; a tile that leaves one CTA per SM is only taken for want of others, and
+        // a plane that already has 4 waves of CTAs (2 per SM) gains nothing from more of them
+        bool two = false;
+        for (int r = 8; r >= 1; r >>= 1) two |= entry_scan_fits2(e, r);
+        for (int r = 8, last = 0; r >= 1; r >>= 1) {
+            if (!(two ? entry_scan_fits2(e, r) : entry_scan_fits(e, r))) continue;
+            if (last && scan_ctas(e, last) >= 8LL * sms) break;
             cands.push_back({0, r});
             last = r;
         }
     }
+    // untimed: 4 rows, or the first candidate where 4 is none
+    if (!cands.empty() && std::find(cands.begin(), cands.end(), std::make_pair(0, 4)) == cands.end())
+        e.rows = cands[0].second;
     if (tc_ok && f->match_form != 0) cands.push_back({1, 4});
     if (cands.size() < 2) return;
     const char *off = getenv("ZB3D_AUTOTUNE");
