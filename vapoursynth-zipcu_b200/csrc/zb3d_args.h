@@ -18,6 +18,7 @@ struct MatchArgs {
     int nbx_al;            // blocks whose x = bs*kx needs no clamp
     int tile_pitch;        // shared tile row pitch in floats (tiled kernel)
     int chunks;            // ceil((2*range+1)/4)
+    int direct;            // scan kernel: 1 = a warp per block row, candidates inserted at once; 0 = 8 warps, queues
     int tiles_x;           // scan kernel: tiles per row; one more column of CTAs takes the clamped blocks
     int2 *list;            // [nby*nbx][8]: (x, y | z << 24)
     float *errs;           // [nby*nbx][8]: distances of the spatial list (radius > 0)

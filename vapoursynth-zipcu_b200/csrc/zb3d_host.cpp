@@ -43,6 +43,7 @@ int pilot_device(const zb3d_pilot *p);
 size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
 bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta);
 bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta);
+int scan_shape(MatchArgs &a, int metric, bool full);
 size_t batch_match_smem(const MatchArgs &m);
 cudaError_t launch_batch(const BatchArgs &b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st);
 cudaError_t filter_precision_init(int dev);
@@ -254,6 +255,7 @@ struct Entry {
     size_t frame_off;              // offset inside one cached source frame [clips][entry planes][h][pitch]
     int form = 0;                  // block matching: 0 FP32 scan, 1 tensor-core bound + exact re-rank
     int rows = 4;                  // block rows per CTA of the tiled FP32 matchers
+    int direct = 0;                // scan kernel: candidates inserted at once (MatchArgs::direct)
 };
 
 // Device scratch of one in-flight frame (the reference's per-stream slot).
@@ -432,6 +434,7 @@ cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, boo
             ma.zero[1] = s.den;
             ma.zero_count = (long long)en.nplanes * f->tw * (long long)en.plane_elems;
         }
+        ma.direct = en.direct;
         const int rows = en.rows;
         bool tiled = (en.bs == 4 || en.bs == 8);
         if (tiled) {
@@ -449,13 +452,17 @@ cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, boo
 // fastest launch configuration of the matching stage for a plane geometry,
 // timed on this GPU.  Every candidate gives bit-identical lists, so the choice
 // never changes results.  Cache file: $ZB3D_TUNE_CACHE, else
-// $XDG_CACHE_HOME/zb3d/tune-v3.txt or ~/.cache/zb3d/tune-v3.txt; one line per key
-// "key form rows".  ZB3D_AUTOTUNE=0 turns the timing off (defaults are used).
+// $XDG_CACHE_HOME/zb3d/tune-v4.txt or ~/.cache/zb3d/tune-v4.txt; one line per key
+// "key form rows direct".  ZB3D_AUTOTUNE=0 turns the timing off (defaults are used).
+struct Shape {
+    int form, rows, direct;  // as in Entry
+};
+
 struct TuneCache {
     std::mutex mu;
     bool loaded = false;
     std::string path;
-    std::map<std::string, std::pair<int, int>> best;
+    std::map<std::string, Shape> best;
 };
 
 TuneCache &tune_cache() {
@@ -467,9 +474,9 @@ std::string tune_path() {
     const char *p = getenv("ZB3D_TUNE_CACHE");
     if (p && *p) return p;
     const char *x = getenv("XDG_CACHE_HOME");
-    if (x && *x) return std::string(x) + "/zb3d/tune-v3.txt";
+    if (x && *x) return std::string(x) + "/zb3d/tune-v4.txt";
     const char *h = getenv("HOME");
-    if (h && *h) return std::string(h) + "/.cache/zb3d/tune-v3.txt";
+    if (h && *h) return std::string(h) + "/.cache/zb3d/tune-v4.txt";
     return "";
 }
 
@@ -479,14 +486,17 @@ void tune_load(TuneCache &c) {
     if (c.path.empty()) return;
     FILE *fp = fopen(c.path.c_str(), "r");
     if (!fp) return;
-    char key[256];
-    int form, rows;
-    while (fscanf(fp, "%255s %d %d", key, &form, &rows) == 3) c.best[key] = {form, rows};
+    char line[512], key[256];
+    Shape v;
+    while (fgets(line, sizeof line, fp)) {
+        v.direct = 0;  // a line may end after the rows
+        if (sscanf(line, "%255s %d %d %d", key, &v.form, &v.rows, &v.direct) >= 3) c.best[key] = v;
+    }
     fclose(fp);
 }
 
-void tune_store(TuneCache &c, const std::string &key, int form, int rows) {
-    c.best[key] = {form, rows};
+void tune_store(TuneCache &c, const std::string &key, const Shape &v) {
+    c.best[key] = v;
     if (c.path.empty()) return;
     const size_t cut = c.path.find_last_of('/');
     if (cut != std::string::npos) {
@@ -496,29 +506,29 @@ void tune_store(TuneCache &c, const std::string &key, int form, int rows) {
     }
     FILE *fp = fopen(c.path.c_str(), "a");
     if (!fp) return;
-    fprintf(fp, "%s %d %d\n", key.c_str(), form, rows);
+    fprintf(fp, "%s %d %d %d\n", key.c_str(), v.form, v.rows, v.direct);
     fclose(fp);
 }
 
-// Whether the scan kernel takes the entry with `rows` block rows per CTA.
-bool entry_scan_fits(const Entry &e, int rows) {
+MatchArgs scan_args(const Entry &e, int direct) {
     MatchArgs t{};
     t.bs = e.bs;
     t.range = e.range;
     t.chunks = (2 * e.range + 1 + 3) / 4;
     t.tile_pitch = 128 + 4 * t.chunks;
-    return scan_rows_fit(t, e.metric, rows);
+    t.direct = direct;
+    t.nbx_al = e.nbx_al;
+    t.nby = e.nby;
+    return t;
 }
 
-// Whether two CTAs of that shape fit an SM's shared memory.
-bool entry_scan_fits2(const Entry &e, int rows) {
-    MatchArgs t{};
-    t.bs = e.bs;
-    t.range = e.range;
-    t.chunks = (2 * e.range + 1 + 3) / 4;
-    t.tile_pitch = 128 + 4 * t.chunks;
-    return scan_rows_fit2(t, e.metric, rows);
+// Whether the scan kernel takes the entry with `rows` block rows per CTA.
+bool entry_scan_fits(const Entry &e, int rows, int direct = 0) {
+    return scan_rows_fit(scan_args(e, direct), e.metric, rows);
 }
+
+// Whether two CTAs of that shape (with queues) fit an SM's shared memory.
+bool entry_scan_fits2(const Entry &e, int rows) { return scan_rows_fit2(scan_args(e, 0), e.metric, rows); }
 
 // CTAs of the scan kernel for the entry.
 long long scan_ctas(const Entry &e, int rows) {
@@ -526,10 +536,12 @@ long long scan_ctas(const Entry &e, int rows) {
     return (long long)((e.nbx_al + nbw - 1) / nbw) * ((e.nby + rows - 1) / rows);
 }
 
-// Chooses e.form / e.rows: FP32 scan with 2 or 4 block rows per CTA (tiled block
-// steps 4 and 8) or, for the scan kernel (ssd, sad), 8 block rows or fewer (its CTAs always
-// have 8 warps; fewer rows split each block's candidate rows, which helps a plane whose CTAs
-// do not fill the GPU), or the tensor-core form (ssd, where eligible), by timing each on a
+// Chooses the entry's matching shape: FP32 scan with 2 or 4 block rows per CTA (tiled block
+// steps 4 and 8) or, for the scan kernel (ssd, sad), 8 block rows or fewer, with queues (8 warps
+// whatever the rows; fewer rows split each block's candidate rows, which helps a plane whose
+// CTAs do not fill the GPU) or with candidates inserted at once (a warp per row, and less shared
+// memory: better where the queues would leave one CTA per SM, and at small ranges, where the
+// tile's load counts most); or the tensor-core form (ssd, where eligible); by timing each on a
 // synthetic plane of the entry's geometry with slot s's buffers.
 void tune_entry(Filter *f, Slot &s, Entry &e) {
     e.rows = 4;
@@ -541,12 +553,13 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     const bool tc_ok = e.metric == M_SSD && f->match_form != 0 && s.tc_ws != nullptr && tc_eligible(ga);
     const bool tiled = e.bs == 4 || e.bs == 8;
     e.form = (f->match_form == 1 && tc_ok) ? 1 : 0;
-    std::vector<std::pair<int, int>> cands;
+    e.direct = 0;
+    std::vector<Shape> cands;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device);
     if (f->match_form != 1 || !tc_ok) {
         if (tiled && !entry_scan_fits(e, 1))
-            for (int r : {2, 4}) cands.push_back({0, r});
+            for (int r : {2, 4}) cands.push_back({0, r, 0});
         // from 8 rows down; a tile that leaves one CTA per SM is only taken for want of others, and
         // a plane that already has 4 waves of CTAs (2 per SM) gains nothing from more of them
         bool two = false;
@@ -554,14 +567,23 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
         for (int r = 8, last = 0; r >= 1; r >>= 1) {
             if (!(two ? entry_scan_fits2(e, r) : entry_scan_fits(e, r))) continue;
             if (last && scan_ctas(e, last) >= 8LL * sms) break;
-            cands.push_back({0, r});
+            cands.push_back({0, r, 0});
             last = r;
         }
     }
-    // untimed: 4 rows, or the first candidate where 4 is none
-    if (!cands.empty() && std::find(cands.begin(), cands.end(), std::make_pair(0, 4)) == cands.end())
-        e.rows = cands[0].second;
-    if (tc_ok && f->match_form != 0) cands.push_back({1, 4});
+    MatchArgs untimed = scan_args(e, 0);
+    untimed.radius = f->radius;
+    if (const int r = cands.empty() ? 0 : scan_shape(untimed, e.metric, false)) {
+        e.rows = r;
+        e.direct = untimed.direct;
+    }
+    // inserted at once: not beside a temporal search, whose accumulators (166 MB of zeros for a
+    // 1080p radius 2 window) such a CTA writes before it starts, with no other CTA's arithmetic
+    // to hide them (three windows in flight: 381 us a window with queues, 391 without)
+    if (!cands.empty() && f->radius == 0)
+        for (int r = 8; r >= 2; r >>= 1)
+            if (entry_scan_fits(e, r, 1)) cands.push_back({0, r, 1});
+    if (tc_ok && f->match_form != 0) cands.push_back({1, 4, 0});
     if (cands.size() < 2) return;
     const char *off = getenv("ZB3D_AUTOTUNE");
     if (off && strcmp(off, "0") == 0) return;
@@ -582,13 +604,13 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     }
     auto it = c.best.find(key);
     if (it != c.best.end()) {
-        const int form = it->second.first, rows = it->second.second;
-        const bool scan = entry_scan_fits(e, 1);
-        if ((form == 0 && !scan && (rows == 2 || rows == 4)) ||
-            (form == 0 && scan && (rows == 1 || rows == 2 || rows == 4 || rows == 8) && entry_scan_fits(e, rows)) ||
-            (form == 1 && tc_ok)) {
-            e.form = form;
-            e.rows = rows;
+        const Shape &v = it->second;
+        const bool scan = entry_scan_fits(e, 1), pow2 = v.rows == 1 || v.rows == 2 || v.rows == 4 || v.rows == 8;
+        if ((v.form == 0 && !scan && (v.rows == 2 || v.rows == 4)) ||
+            (v.form == 0 && scan && pow2 && entry_scan_fits(e, v.rows, v.direct)) || (v.form == 1 && tc_ok)) {
+            e.form = v.form;
+            e.rows = v.rows;
+            e.direct = v.form == 0 && scan && v.direct != 0;
         }
         return;
     }
@@ -607,19 +629,21 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     for (int t = 0; ok && t < f->tw; ++t)
         ok = cudaMemcpy(s.d_src + e.src_off + (size_t)t * e.plane_elems, host.data(), host.size() * sizeof(float),
                         cudaMemcpyHostToDevice) == cudaSuccess;
-    float best_ms = 3.0e38f;
-    int bform = -1, brows = e.rows;
-    std::vector<std::pair<float, std::pair<int, int>>> times;
+    float best_ms = 3.0e38f;  // of the shapes with queues, and the tensor-core form
+    Shape best{-1, e.rows, 0};
+    std::vector<std::pair<float, Shape>> times;
     for (const auto &cand : cands) {
         if (!ok) break;
         Entry t = e;
-        t.form = cand.first;
-        t.rows = cand.second;
+        t.form = cand.form;
+        t.rows = cand.rows;
+        t.direct = cand.direct;
         float lo = 3.0e38f;
         bool good = true;
         for (int it2 = 0; it2 < 4 && good; ++it2) {
             good = cudaEventRecord(a, s.st) == cudaSuccess &&
-                   run_match(f, s, t, s.d_src + e.src_off) == cudaSuccess && cudaEventRecord(b, s.st) == cudaSuccess &&
+                   run_match(f, s, t, s.d_src + e.src_off, true) == cudaSuccess &&  // with the accumulators' zeros
+                   cudaEventRecord(b, s.st) == cudaSuccess &&
                    cudaEventSynchronize(b) == cudaSuccess;
             float ms = 0.0f;
             if (good && cudaEventElapsedTime(&ms, a, b) == cudaSuccess && it2 > 0) lo = std::min(lo, ms);
@@ -628,7 +652,7 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
             cudaGetLastError();
             continue;
         }
-        if (lo < best_ms) best_ms = lo;
+        if (!cand.direct && lo < best_ms) best_ms = lo;
         times.push_back({lo, cand});
     }
     // The first candidate within 20% of the fastest: fewer block rows per CTA make one plane's
@@ -637,12 +661,22 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     // block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3 streams).
     // A plane that leaves SMs without a CTA even at one row takes the fastest.
     const float slack = entry_scan_fits(e, 1) && scan_ctas(e, 1) > sms ? 1.2f : 1.0f;
+    float chosen_ms = 3.0e38f;
     for (const auto &t : times)
-        if (bform < 0 && t.first <= slack * best_ms) {
-            bform = t.second.first;
-            brows = t.second.second;
+        if (best.form < 0 && !t.second.direct && t.first <= slack * best_ms) {
+            best = t.second;
+            chosen_ms = t.first;
         }
-    ok = ok && bform >= 0;
+    // Inserted at once: where it is clearly faster alone.  With other streams beside it a few
+    // per cent do not last (1080p block_step 4, bm_range 12, 4% alone: two passes 1301 us with
+    // queues, 1312 without; block_step 8, bm_range 9, 13% alone: Wiener 256 and 247 us).
+    chosen_ms *= 0.93f;
+    for (const auto &t : times)
+        if (t.second.direct && t.first < chosen_ms) {
+            best = t.second;
+            chosen_ms = t.first;
+        }
+    ok = ok && best.form >= 0;
     if (a) cudaEventDestroy(a);
     if (b) cudaEventDestroy(b);
     if (s.tc_stats) cudaMemset(s.tc_stats, 0, 4 * sizeof(unsigned long long));
@@ -650,9 +684,10 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
         cudaGetLastError();
         return;
     }
-    e.form = bform;
-    e.rows = brows;
-    tune_store(c, key, bform, brows);
+    e.form = best.form;
+    e.rows = best.rows;
+    e.direct = best.direct;
+    tune_store(c, key, best);
 }
 
 cudaEvent_t prof_event(Filter *f, std::vector<cudaEvent_t> &v, cudaStream_t st) {

@@ -445,9 +445,9 @@ __global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps *
             const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
             if (cy < m.nby) warp_block<M_SSD>(m, m.nbx - 1, cy);
         } else if (m.bs == 4) {
-            scan_tile<M_SSD, true, 4>(m, bx, by, kBatchMatchRows, dyn);
+            scan_tile<M_SSD, true, 4, true>(m, bx, by, kBatchMatchRows, dyn);
         } else {
-            scan_tile<M_SSD, false, 8>(m, bx, by, kBatchMatchRows, dyn);
+            scan_tile<M_SSD, false, 8, true>(m, bx, by, kBatchMatchRows, dyn);
         }
         __threadfence();  // each thread's list stores before the tile's count
         __syncthreads();

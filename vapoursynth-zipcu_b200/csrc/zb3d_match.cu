@@ -133,10 +133,10 @@ __global__ void __launch_bounds__(128) zb_match_column(MatchArgs a) {
 }
 
 // Spatial SSD / SAD matching at block_step 4 and 8 (scan_tile), `rows` block rows per CTA of 8
-// warps.  Where the plane's width leaves a clamped last block column, one more column of CTAs
+// warps (QUEUE) or `rows` warps.  Where the plane's width leaves a clamped last block column, one more column of CTAs
 // scans it, a warp per block, instead of a launch of its own (11 to 17 us, most of it the
 // latency of one warp per block).
-template <int M, bool SHARED, int BS>
+template <int M, bool SHARED, int BS, bool QUEUE>
 __global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a, int rows) {
     extern __shared__ __align__(16) float tile[];
     zero_slice(a.zero, a.zero_count, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a,
         if (warp < rows && by < a.nby) warp_block<M>(a, a.nbx - 1, by);
         return;
     }
-    scan_tile<M, SHARED, BS>(a, blockIdx.x, blockIdx.y, rows, tile);
+    scan_tile<M, SHARED, BS, QUEUE>(a, blockIdx.x, blockIdx.y, rows, tile);
 }
 
 // Spatial matching for block steps the tiled kernels do not take (and the blocks the
@@ -348,15 +348,41 @@ bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta) {
     return scan_rows_fit(a, metric, rows_per_cta) && scan_smem_bytes(a, rows_per_cta) <= kSmemOptIn / 2;
 }
 
+// The scan's shape without a timing: sets a.direct and returns the block rows per CTA (0: the
+// kernel takes no shape of the entry).  full: other planes fill the GPU beside this one.
+// 3840x2160 ssd, us (block_step 4 / 8; d8 and d4: inserted at once with 8 and 4 rows, q8 .. q1: queues):
+//   bm_range  9:  d8  602 /  293, d4  573 /  308, q8  625 /  370, q4  689 /  339
+//   bm_range 16:  d8 1618 /  994, d4 1637 /  931, q8 1890 /  907, q4 1702 /  988, q2 1861 /  918
+//   bm_range 24:  d8 4373 / 2064, d4 3879 / 1910, q8 3818 / 1825, q4 3955 / 1932, q1 4087 / 1989
+// so with CTAs enough (and no temporal search, see tune_entry): at once while two CTAs of 8 rows
+// fit an SM, then queues with the most rows
+// (2 at least) that two CTAs fit with, then queues with the most rows.  With fewer CTAs than two
+// per SM the split of the candidate rows counts most (640x480 at block_step 8, bm_range 9: d8 61,
+// d4 51, q4 47, q2 38, q1 32; 320x240 at 4, bm_range 12: d8 92, d4 75, q4 65, q2 42, q1 40): queues
+// with 4 rows, which cost the other streams less than more ranges would.
+int scan_shape(MatchArgs &a, int metric, bool full) {
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    full = full || (long long)scan_tiles_x(a) * ((a.nby + 3) / 4) >= 2LL * sms;
+    a.direct = 1;
+    if (full && a.radius == 0 && scan_rows_fit2(a, metric, 8)) return 8;
+    a.direct = 0;
+    for (int r = full ? 8 : 4; r >= (full ? 2 : 1); r >>= 1)
+        if (scan_rows_fit2(a, metric, r)) return r;
+    for (int r = full ? 8 : 4; r >= 1; r >>= 1)
+        if (scan_rows_fit(a, metric, r)) return r;
+    return 0;
+}
+
 template <int M, bool SHARED, int BS>
 static cudaError_t launch_scan_t(const MatchArgs &a, int rows, cudaStream_t st) {
-    auto k = zb_match_scan<M, SHARED, BS>;
+    auto k = a.direct ? zb_match_scan<M, SHARED, BS, false> : zb_match_scan<M, SHARED, BS, true>;
     // the same limit at every launch: a limit of this launch's size would race with other
     // threads' launches of the same kernel
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptIn);
     if (e != cudaSuccess) return e;
     const int gx = a.tiles_x + (a.nbx_al != a.nbx ? 1 : 0), gy = (a.nby + rows - 1) / rows;
-    k<<<dim3(gx, gy), kScanWarps * 32, scan_smem_bytes(a, rows), st>>>(a, rows);
+    k<<<dim3(gx, gy), (a.direct ? rows : kScanWarps) * 32, scan_smem_bytes(a, rows), st>>>(a, rows);
     return cudaGetLastError();
 }
 

@@ -1,8 +1,9 @@
 // Spatial SSD / SAD matching of one shared-memory tile, used by the per-plane kernel
 // (zb3d_match.cu) and by the batch kernel (zb3d_kernels.cu).
 //
-// A CTA has kScanWarps warps: rows_per_cta block rows times `split` ranges of candidate
-// rows.  A warp covers one row of reference blocks and one of the ranges; lane k's half
+// A CTA has a warp per block row (candidates inserted into the lists at once), or kScanWarps
+// warps: rows_per_cta block rows times `split` ranges of candidate rows (candidates queued).  A
+// warp covers one row of reference blocks and one of the ranges; lane k's half
 // block starts at tile column 4k (SHARED, block_step 4: block k = lanes k, k+1) or, in
 // pair mode (block_step 8), block b = lanes 2b, 2b+1.
 //
@@ -21,11 +22,13 @@
 // bm_range <= 15) every other offset is an immediate.
 //
 // What bounds it: the FMA pipe, 72 cycles of it per warp and candidate (16 subtractions and 16
-// multiply-adds of two cycles each, and the joins).  1920x1080, block_step 4, bm_range 12:
-// 326 -> 289 us, 200 -> 169 M instructions, FMA pipe busy 73% of active cycles (69% before);
-// the 544 CTAs are 1.84 waves, which leaves 12% of the SMs' time idle when the plane runs
-// alone.  959x541 sad: 136 + 17 -> about 100 us (packed differences, the clamped column in the
-// same launch).  77x53 at block_step 8: 47 + 11 -> 23 us with 8 ranges per block row.
+// multiply-adds of two cycles each, and the joins); with queues 73% of active cycles at 1920x1080,
+// block_step 4, bm_range 12, whose 544 CTAs are 1.84 waves.  The queues' 32 KB decide how many
+// CTAs share an SM, so where that costs more than they save candidates are inserted at once:
+// 1080p us at block_step 4 / 8, inserted at once and queued (8 rows, ssd): bm_range 9 174 / 97 and
+// 185 / 119, bm_range 12 275 / 149 and 284 / 175, bm_range 24 1184 / 601 and 1049 / 544.  Small
+// planes take queues for their ranges of candidate rows: 320x240 at block_step 4, bm_range 12: 92
+// at once, 40 with 8 ranges.  scan_shape (zb3d_match.cu) has the rule, and the autotuner times both.
 #pragma once
 #include "zb3d_match.cuh"
 
@@ -47,7 +50,7 @@ __device__ __forceinline__ float2 f4lo(const float4 &v) { return make_float2(v.x
 __device__ __forceinline__ float2 f4hi(const float4 &v) { return make_float2(v.z, v.w); }
 
 // ---------------------------------------------------------------------------
-// Pending candidates.  A candidate below the list's last error is not inserted at once:
+// Pending candidates (QUEUE).  A candidate below the list's last error is not inserted at once:
 // the lane appends it to its own queue in shared memory, and the warp drains all its queues
 // together when one of them could overflow, and at the end.  With immediate insertion a
 // warp ran the 38-instruction insertion at about 380 of the 625 candidates of bm_range 12,
@@ -165,10 +168,29 @@ __device__ __forceinline__ void scan_step(const float *pc, int pp_rt, int g_rt, 
     }
 }
 
+// Displacement at `pos` of the joined error err: queued, or inserted at once, where it is below
+// the list's last error.
+template <bool QUEUE>
+__device__ __forceinline__ void scan_take(float err, int pos, unsigned &end, float (&e)[8], int (&q)[8]) {
+    if (err < e[7]) {
+        if constexpr (QUEUE) {
+            pend_store(end, err, pos);
+            end += 256;
+        } else {
+            top8_insert(e, q, err, pos);
+        }
+    }
+}
+
+template <bool QUEUE>
+__device__ __forceinline__ void scan_vote(unsigned base, unsigned &end, float (&e)[8], int (&q)[8]) {
+    if constexpr (QUEUE)
+        if (__any_sync(kFull, end > base + kPendFull)) pend_drain(base, end, e, q);
+}
+
 // The step, then its finished displacements C0 .. C1 - 1 joined with the other half block
-// and appended where they are below the list's last error.  pos: packed position of
-// displacement 4m - 3.
-template <int M, bool SHARED, int GF, bool FIRST, int SMAX, int C0, int C1>
+// and taken.  pos: packed position of displacement 4m - 3.
+template <int M, bool SHARED, int GF, bool QUEUE, bool FIRST, int SMAX, int C0, int C1>
 __device__ __forceinline__ void scan_step_append(const float *pc, int pp, int g, const float2 (&nc)[4][4],
                                                  float (&st)[4], int pos, unsigned base, unsigned &end, float (&e)[8],
                                                  int (&q)[8]) {
@@ -178,16 +200,12 @@ __device__ __forceinline__ void scan_step_append(const float *pc, int pp, int g,
     for (int c = C0; c < C1; ++c)
         err[c] += SHARED ? __shfl_down_sync(kFull, err[c], 1) : __shfl_xor_sync(kFull, err[c], 1);
 #pragma unroll
-    for (int c = C0; c < C1; ++c)
-        if (err[c] < e[7]) {
-            pend_store(end, err[c], pos + c);
-            end += 256;
-        }
-    if (__any_sync(kFull, end > base + kPendFull)) pend_drain(base, end, e, q);
+    for (int c = C0; c < C1; ++c) scan_take<QUEUE>(err[c], pos + c, end, e, q);
+    scan_vote<QUEUE>(base, end, e, q);
 }
 
 // Two whole steps with one vote.
-template <int M, bool SHARED, int GF>
+template <int M, bool SHARED, int GF, bool QUEUE>
 __device__ __forceinline__ void scan_two_steps(const float *pc, int pp, int g, const float2 (&nc)[4][4],
                                                float (&st)[4], int pos, unsigned base, unsigned &end, float (&e)[8],
                                                int (&q)[8]) {
@@ -198,22 +216,19 @@ __device__ __forceinline__ void scan_two_steps(const float *pc, int pp, int g, c
     for (int c = 0; c < 8; ++c)
         err[c >> 2][c & 3] += SHARED ? __shfl_down_sync(kFull, err[c >> 2][c & 3], 1) : __shfl_xor_sync(kFull, err[c >> 2][c & 3], 1);
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-        if (err[c >> 2][c & 3] < e[7]) {
-            pend_store(end, err[c >> 2][c & 3], pos + c);
-            end += 256;
-        }
-    if (__any_sync(kFull, end > base + kPendFull)) pend_drain(base, end, e, q);
+    for (int c = 0; c < 8; ++c) scan_take<QUEUE>(err[c >> 2][c & 3], pos + c, end, e, q);
+    scan_vote<QUEUE>(base, end, e, q);
 }
 
-// Bytes of dynamic shared memory: the two copies of the tile, then the queues.
+// Bytes of dynamic shared memory: the two copies of the tile, then the queues (none where
+// candidates are inserted at once).
 inline size_t scan_tile_bytes(const MatchArgs &a, int rows_per_cta) {
     return (size_t)((rows_per_cta - 1) * a.bs + 2 * a.range + 8) * 8 * tile2_g(a.tile_pitch, tile2_fixed(a.chunks)) *
            sizeof(float);
 }
 
 inline size_t scan_smem_bytes(const MatchArgs &a, int rows_per_cta) {
-    return scan_tile_bytes(a, rows_per_cta) + (size_t)kScanWarps * kPendBytes;
+    return scan_tile_bytes(a, rows_per_cta) + (a.direct ? 0 : (size_t)kScanWarps * kPendBytes);
 }
 
 // CTA `part` of `parts` clears its share of the accumulators (16-byte stores; the arrays start
@@ -238,16 +253,17 @@ inline int scan_tiles_x(const MatchArgs &a) {
 
 // One tile: block columns [31 bx, 31 bx + 31) (SHARED) or [16 bx, ...), block rows
 // [rows by, rows by + rows); `tile` is the dynamic shared memory (scan_smem_bytes).
-// split = kScanWarps / rows ranges of candidate rows per block row: with fewer rows per CTA a
-// plane gives more CTAs, which is what fills the GPU for small planes.  The ranges' lists
-// are merged in row order at the end, a later range's entries inserted (strict less) after
-// the earlier ranges', which is the list of one scan.
-template <int M, bool SHARED, int BS, bool FIXED>
+// QUEUE: kScanWarps warps, split = kScanWarps / rows ranges of candidate rows per block row:
+// with fewer rows per CTA a plane gives more CTAs, which is what fills the GPU for small planes.
+// The ranges' lists are merged in row order at the end, a later range's entries inserted
+// (strict less) after the earlier ranges', which is the list of one scan.  Else: a warp per block
+// row, no queues and no ranges.
+template <int M, bool SHARED, int BS, bool FIXED, bool QUEUE>
 __device__ __forceinline__ void scan_tile_g(const MatchArgs &a, int bx, int by_cta, int rows, float *tile) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NBW = SHARED ? 31 : 16;
     constexpr int GF = FIXED ? kTile2G : 0;
-    const int split = kScanWarps / rows;
+    const int warps = QUEUE ? kScanWarps : rows, split = QUEUE ? kScanWarps / rows : 1;
     const int R = a.range, W = a.w, H = a.h, tp = a.tile_pitch;
     const int g = tile2_g(tp, FIXED), pp = 8 * g;
     const int kx0 = bx * NBW;
@@ -266,7 +282,7 @@ __device__ __forceinline__ void scan_tile_g(const MatchArgs &a, int bx, int by_c
         // columns outside the image are +inf: every candidate that touches one has an
         // infinite (or NaN) distance and never enters a list, so the scan needs no bounds tests
         const int gx0 = x0 - R;
-        for (int t = warp; t < nrows; t += kScanWarps) {
+        for (int t = warp; t < nrows; t += warps) {
             const float *srow = plane + (long long)(r0 + t) * a.pitch;
             float *de = tE + (t >> 1) * pp + (t & 1);
             float *dq = t > 0 ? tO + ((t - 1) >> 1) * pp + ((t - 1) & 1) : nullptr;
@@ -330,25 +346,25 @@ __device__ __forceinline__ void scan_tile_g(const MatchArgs &a, int bx, int by_c
             const float *pc = ((t0 & 1) ? tO + ((t0 - 1) >> 1) * pp : tE + (t0 >> 1) * pp) + uo;
             int pos = pack_pos(0, row) + (xb - R - 3);
             float st[4];
-            scan_step_append<M, SHARED, GF, true, 3, 3, 4>(pc, pp, g, nc, st, pos, base, end, e, q);
+            scan_step_append<M, SHARED, GF, QUEUE, true, 3, 3, 4>(pc, pp, g, nc, st, pos, base, end, e, q);
             int m = 1;
             for (; m + 1 < (R + 1) / 2; m += 2) {
-                scan_two_steps<M, SHARED, GF>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
+                scan_two_steps<M, SHARED, GF, QUEUE>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
                 pc += 8;
                 pos += 8;
             }
             if (m < (R + 1) / 2) {
                 pc += 4;
                 pos += 4;
-                scan_step_append<M, SHARED, GF, false, 3, 0, 4>(pc, pp, g, nc, st, pos, base, end, e, q);
+                scan_step_append<M, SHARED, GF, QUEUE, false, 3, 0, 4>(pc, pp, g, nc, st, pos, base, end, e, q);
             }
             // displacement 2R is the first of its step (R even) or the last of the step before
             if (R & 1)
-                scan_step_append<M, SHARED, GF, false, -2, 0, 2>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
+                scan_step_append<M, SHARED, GF, QUEUE, false, -2, 0, 2>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
             else
-                scan_step_append<M, SHARED, GF, false, 0, 0, 4>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
+                scan_step_append<M, SHARED, GF, QUEUE, false, 0, 0, 4>(pc + 4, pp, g, nc, st, pos + 4, base, end, e, q);
         }
-        pend_drain(base, end, e, q);
+        if constexpr (QUEUE) pend_drain(base, end, e, q);
     }
     // merge of the ranges, in order: range sp takes the list of range sp + k
     for (int k = 1; k < split; k <<= 1) {
@@ -374,12 +390,12 @@ __device__ __forceinline__ void scan_tile_g(const MatchArgs &a, int bx, int by_c
 }
 
 // The tile with the fixed half-plane size where the displacements allow it.
-template <int M, bool SHARED, int BS>
+template <int M, bool SHARED, int BS, bool QUEUE>
 __device__ __forceinline__ void scan_tile(const MatchArgs &a, int bx, int by_cta, int rows, float *tile) {
     if (tile2_fixed(a.chunks))
-        scan_tile_g<M, SHARED, BS, true>(a, bx, by_cta, rows, tile);
+        scan_tile_g<M, SHARED, BS, true, QUEUE>(a, bx, by_cta, rows, tile);
     else
-        scan_tile_g<M, SHARED, BS, false>(a, bx, by_cta, rows, tile);
+        scan_tile_g<M, SHARED, BS, false, QUEUE>(a, bx, by_cta, rows, tile);
 }
 
 }  // namespace zb

@@ -34,6 +34,7 @@ namespace zb {
 
 cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st);
 size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
+int scan_shape(MatchArgs &a, int metric, bool full);
 cudaError_t launch_filter(const FilterArgs &a, bool final_, int t2d, int t1d, cudaStream_t st);
 cudaError_t launch_finish(const unsigned long long *num, const unsigned long long *den, long long acc_plane_stride,
                           long long acc_frame_stride, int w, int h, int pitch, int nplanes, int tw,
@@ -153,13 +154,18 @@ extern "C" int zb3d_bm3d_plane_noalloc(const float *d_src, float *d_dst, int wid
     ma.zero[1] = den;
     ma.zero_count = (long long)pixels;
     bool tiled = block_step == 4 || block_step == 8;
+    int rows = 4;
     if (tiled) {
         MatchArgs t = ma;
         t.chunks = (2 * bm_range + 1 + 3) / 4;
         t.tile_pitch = 128 + 4 * t.chunks;
         tiled = match_tile_bytes(t, 4) <= 200 * 1024;
+        if (const int r = scan_shape(t, M_SSD, false)) {
+            rows = r;
+            ma.direct = t.direct;
+        }
     }
-    if (e == cudaSuccess) e = launch_match(ma, M_SSD, 4, tiled, st);
+    if (e == cudaSuccess) e = launch_match(ma, M_SSD, rows, tiled, st);
 
     FilterArgs fa{};
     fa.src = d_src;
