@@ -8,6 +8,10 @@ enum Metric { M_SSD = 0, M_SAD = 1, M_ZSSD = 2, M_ZSAD = 3, M_SSD_NORM = 4 };
 
 // Block matching of one plane entry.  Reference blocks sit at
 // x = min(bs*kx, w-8), y = min(bs*ky, h-8) (vszipcu src/bm3d.cu:585-595).
+// A kernel argument of at most 128 bytes: with a larger one nvcc compiles every kernel that takes
+// it to other registers (sad scan from global memory 126 -> 120, general temporal search of ssd
+// with 8 entries 228 -> 464 bytes of spills), and those were up to 18% slower.  What only the
+// launchers or one kernel want is in MatchJob.
 struct MatchArgs {
     const float *frames;   // matching plane of window frame t at frames + t*fstride
     long long fstride;
@@ -18,15 +22,9 @@ struct MatchArgs {
     int nbx_al;            // blocks whose x = bs*kx needs no clamp
     int tile_pitch;        // shared tile row pitch in floats (tiled kernel)
     int chunks;            // ceil((2*range+1)/4)
-    int direct;            // scan kernel: 1 = a warp per block row, candidates inserted at once; 0 = 8 warps, queues
     int tiles_x;           // scan kernel: tiles per row; one more column of CTAs takes the clamped blocks
     int2 *list;            // [nby*nbx][8]: (x, y | z << 24)
     float *errs;           // [nby*nbx][8]: distances of the spatial list (radius > 0)
-    // Accumulators that start from zero after the matching (null: none): two arrays of
-    // zero_count 64-bit words.  The scan kernel writes the zeros itself, its stores being free
-    // beside the arithmetic; before the other matchers they are cleared by memset nodes.
-    unsigned long long *zero[2];
-    long long zero_count;
     int self_incl;         // 1: insert the block itself here (radius 0)
     int gen_mode;          // generic kernel: 0 = every block, 2 = the blocks listed in tc_ws
                            // (fallbacks of the tensor-core form)
@@ -40,6 +38,22 @@ struct MatchArgs {
                                   // polls of the block and issuer warps [8], [10], TMEM load cycles
                                   // and count [11], [13], pass-1 / pass-2 / done-wait cycles [12], [14], [15]; then for tile (1, 1) a per-job trace
                                   // [job][3] (issued, completion seen, slot freed), at most 64 jobs
+};
+
+static_assert(sizeof(MatchArgs) <= 128, "see above");
+
+// Accumulators that start from zero after the matching (null: none): two arrays of `count`
+// 64-bit words.  The scan kernel writes the zeros itself, its stores being free beside the
+// arithmetic; before the other matchers they are cleared by memset nodes.
+struct ZeroArgs {
+    unsigned long long *acc[2];
+    long long count;
+};
+
+// What launch_match takes.
+struct MatchJob : MatchArgs {
+    ZeroArgs zero;
+    int direct;            // scan kernel: 1 = a warp per block row, candidates inserted at once; 0 = 8 warps, queues
 };
 
 constexpr int kTcWsList = 8;
@@ -64,6 +78,7 @@ struct FilterArgs {
 // match tiles first (all entries), then filter chunks (all entries).
 struct BatchEntry {
     MatchArgs m;                      // tile_pitch, chunks and self_incl set; bs 4 or 8
+    ZeroArgs zero;
     FilterArgs f;
     int tiles_x;                      // match items per tile row: m.tiles_x tiles, and one for the
                                       // clamped last block column where there is one

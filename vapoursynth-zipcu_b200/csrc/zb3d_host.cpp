@@ -34,17 +34,17 @@
 
 namespace zb {
 
-cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st);
+cudaError_t launch_match(MatchJob a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st);
 bool tc_eligible(const MatchArgs &a);
 cudaError_t launch_match_tc(const MatchArgs &a, cudaStream_t st);
 cudaError_t launch_tc_fallback(MatchArgs a, cudaStream_t st);
 int tc_debug_cols(const MatchArgs &a);
 int pilot_device(const zb3d_pilot *p);
 size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
-bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta);
-bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta);
-int scan_shape(MatchArgs &a, int metric, bool full);
-size_t batch_match_smem(const MatchArgs &m);
+bool scan_rows_fit(const MatchJob &a, int metric, int rows_per_cta);
+bool scan_rows_fit2(const MatchJob &a, int metric, int rows_per_cta);
+int scan_shape(MatchJob &a, int metric, bool full);
+size_t batch_match_smem(const MatchJob &m);
 cudaError_t launch_batch(const BatchArgs &b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st);
 cudaError_t filter_precision_init(int dev);
 size_t filter_precision_stack_floats(long long nblocks);
@@ -255,7 +255,7 @@ struct Entry {
     size_t frame_off;              // offset inside one cached source frame [clips][entry planes][h][pitch]
     int form = 0;                  // block matching: 0 FP32 scan, 1 tensor-core bound + exact re-rank
     int rows = 4;                  // block rows per CTA of the tiled FP32 matchers
-    int direct = 0;                // scan kernel: candidates inserted at once (MatchArgs::direct)
+    int direct = 0;                // scan kernel: candidates inserted at once (MatchJob::direct)
 };
 
 // Device scratch of one in-flight frame (the reference's per-stream slot).
@@ -411,7 +411,7 @@ bool alloc_slot(Filter *f, Slot &s) {
 // Block matching of one entry into the slot's match list.
 // clear: the accumulators of the entry start from zero after it.
 cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, bool clear = false) {
-        MatchArgs ma{};
+        MatchJob ma{};
         ma.frames = src;  // clip 0, plane 0: the matching plane of every window frame
         ma.fstride = (long long)en.plane_elems;
         ma.w = en.w;
@@ -430,9 +430,9 @@ cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, boo
         ma.tc_ws = en.form == 1 ? s.tc_ws : nullptr;  // null: the FP32 scan
         ma.tc_stats = s.tc_stats;
         if (clear) {
-            ma.zero[0] = s.num;
-            ma.zero[1] = s.den;
-            ma.zero_count = (long long)en.nplanes * f->tw * (long long)en.plane_elems;
+            ma.zero.acc[0] = s.num;
+            ma.zero.acc[1] = s.den;
+            ma.zero.count = (long long)en.nplanes * f->tw * (long long)en.plane_elems;
         }
         ma.direct = en.direct;
         const int rows = en.rows;
@@ -510,8 +510,8 @@ void tune_store(TuneCache &c, const std::string &key, const Shape &v) {
     fclose(fp);
 }
 
-MatchArgs scan_args(const Entry &e, int direct) {
-    MatchArgs t{};
+MatchJob scan_args(const Entry &e, int direct) {
+    MatchJob t{};
     t.bs = e.bs;
     t.range = e.range;
     t.chunks = (2 * e.range + 1 + 3) / 4;
@@ -571,7 +571,7 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
             last = r;
         }
     }
-    MatchArgs untimed = scan_args(e, 0);
+    MatchJob untimed = scan_args(e, 0);
     untimed.radius = f->radius;
     if (const int r = cands.empty() ? 0 : scan_shape(untimed, e.metric, false)) {
         e.rows = r;
@@ -1012,7 +1012,7 @@ bool batch_eligible(const Filter *f, const Entry &en) {
         en.form != 0)
         return false;
     if (en.t2d != 0 || en.t1d != 0) return false;
-    MatchArgs m{};
+    MatchJob m{};
     m.bs = en.bs;
     m.range = en.range;
     m.chunks = (2 * en.range + 1 + 3) / 4;
@@ -1212,9 +1212,9 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
                 m.tile_pitch = 128 + 4 * m.chunks;
                 m.list = list;
                 m.self_incl = 1;
-                m.zero[0] = num;  // cleared by the match items, which the filter chunks wait for
-                m.zero[1] = den;
-                m.zero_count = (long long)en.nplanes * (long long)en.plane_elems;
+                B.zero.acc[0] = num;  // cleared by the match items, which the filter chunks wait for
+                B.zero.acc[1] = den;
+                B.zero.count = (long long)en.nplanes * (long long)en.plane_elems;
                 FilterArgs &fa = B.f;
                 fa.src = src;
                 fa.plane_stride = (long long)en.plane_elems;
@@ -1240,7 +1240,7 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
                 B.filter_items = (int)((en.nblocks + kBatchGroups - 1) / kBatchGroups);
                 B.first_match = nm;
                 nm += B.match_items;
-                smem = std::max(smem, batch_match_smem(m));
+                smem = std::max(smem, batch_match_smem(MatchJob{m}));
             }
             long long nf = nm;
             for (int i = 0; i < n; ++i) {

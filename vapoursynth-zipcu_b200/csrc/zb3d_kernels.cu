@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps *
         const MatchArgs &m = E.m;
         const int local = (int)(item - E.first_match);
         const int bx = local % E.tiles_x, by = local / E.tiles_x;
-        zero_slice(m.zero, m.zero_count, local, E.match_items);
+        zero_slice(E.zero, local, E.match_items);
         if (bx == m.tiles_x) {  // the clamped last block column
             const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
             if (cy < m.nby) warp_block<M_SSD>(m, m.nbx - 1, cy);
@@ -558,7 +558,7 @@ cudaError_t launch_finish(const unsigned long long *num, const unsigned long lon
 }
 
 // Bytes of dynamic shared memory a batch entry's matching needs (kBatchMatchRows block rows).
-size_t batch_match_smem(const MatchArgs &m) { return scan_smem_bytes(m, kBatchMatchRows); }
+size_t batch_match_smem(const MatchJob &m) { return scan_smem_bytes(m, kBatchMatchRows); }
 
 template <class K>
 static cudaError_t launch_batch_k(K k, const BatchArgs &b, long long items, int threads, size_t smem,

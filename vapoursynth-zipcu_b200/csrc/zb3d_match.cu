@@ -137,9 +137,9 @@ __global__ void __launch_bounds__(128) zb_match_column(MatchArgs a) {
 // scans it, a warp per block, instead of a launch of its own (11 to 17 us, most of it the
 // latency of one warp per block).
 template <int M, bool SHARED, int BS, bool QUEUE>
-__global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a, int rows) {
+__global__ void __launch_bounds__(kScanWarps * 32, 2) zb_match_scan(MatchArgs a, ZeroArgs zero, int rows) {
     extern __shared__ __align__(16) float tile[];
-    zero_slice(a.zero, a.zero_count, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
+    zero_slice(zero, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
     if ((int)blockIdx.x == a.tiles_x) {
         const int warp = threadIdx.x >> 5, by = blockIdx.y * rows + warp;
         if (warp < rows && by < a.nby) warp_block<M>(a, a.nbx - 1, by);
@@ -338,13 +338,13 @@ static cudaError_t launch_tiled_t(const MatchArgs &a, int rows_per_cta, cudaStre
 
 // Whether the scan kernel takes an entry with this many block rows per CTA: ssd and sad at
 // block_step 4 and 8, a tile that fits shared memory.
-bool scan_rows_fit(const MatchArgs &a, int metric, int rows_per_cta) {
+bool scan_rows_fit(const MatchJob &a, int metric, int rows_per_cta) {
     if ((metric != M_SSD && metric != M_SAD) || (a.bs != 4 && a.bs != 8)) return false;
     return scan_smem_bytes(a, rows_per_cta) <= kSmemOptIn;
 }
 
 // Whether two such CTAs share an SM (227 KB, 1 KB of it reserved per CTA).
-bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta) {
+bool scan_rows_fit2(const MatchJob &a, int metric, int rows_per_cta) {
     return scan_rows_fit(a, metric, rows_per_cta) && scan_smem_bytes(a, rows_per_cta) <= kSmemOptIn / 2;
 }
 
@@ -360,7 +360,7 @@ bool scan_rows_fit2(const MatchArgs &a, int metric, int rows_per_cta) {
 // per SM the split of the candidate rows counts most (640x480 at block_step 8, bm_range 9: d8 61,
 // d4 51, q4 47, q2 38, q1 32; 320x240 at 4, bm_range 12: d8 92, d4 75, q4 65, q2 42, q1 40): queues
 // with 4 rows, which cost the other streams less than more ranges would.
-int scan_shape(MatchArgs &a, int metric, bool full) {
+int scan_shape(MatchJob &a, int metric, bool full) {
     int sms = 148, dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     full = full || (long long)scan_tiles_x(a) * ((a.nby + 3) / 4) >= 2LL * sms;
@@ -375,27 +375,27 @@ int scan_shape(MatchArgs &a, int metric, bool full) {
 }
 
 template <int M, bool SHARED, int BS>
-static cudaError_t launch_scan_t(const MatchArgs &a, int rows, cudaStream_t st) {
+static cudaError_t launch_scan_t(const MatchJob &a, int rows, cudaStream_t st) {
     auto k = a.direct ? zb_match_scan<M, SHARED, BS, false> : zb_match_scan<M, SHARED, BS, true>;
     // the same limit at every launch: a limit of this launch's size would race with other
     // threads' launches of the same kernel
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptIn);
     if (e != cudaSuccess) return e;
     const int gx = a.tiles_x + (a.nbx_al != a.nbx ? 1 : 0), gy = (a.nby + rows - 1) / rows;
-    k<<<dim3(gx, gy), (a.direct ? rows : kScanWarps) * 32, scan_smem_bytes(a, rows), st>>>(a, rows);
+    k<<<dim3(gx, gy), (a.direct ? rows : kScanWarps) * 32, scan_smem_bytes(a, rows), st>>>(a, a.zero, rows);
     return cudaGetLastError();
 }
 
 // Block rows per CTA of the scan: the asked power of two, or fewer where its tile does not
 // fit; 0 where none does.
-static int scan_rows(const MatchArgs &a, int metric, int rows) {
+static int scan_rows(const MatchJob &a, int metric, int rows) {
     int r = rows >= 8 ? 8 : rows >= 4 ? 4 : rows >= 2 ? 2 : 1;
     while (r > 0 && !scan_rows_fit(a, metric, r)) r >>= 1;
     return r;
 }
 
 template <int M>
-static cudaError_t launch_tiled_m(MatchArgs a, int rows_per_cta, cudaStream_t st) {
+static cudaError_t launch_tiled_m(MatchJob a, int rows_per_cta, cudaStream_t st) {
     if constexpr (M == M_SSD || M == M_SAD) {
         if (const int rows = scan_rows(a, M, rows_per_cta)) {
             a.tiles_x = scan_tiles_x(a);
@@ -469,17 +469,17 @@ cudaError_t launch_tc_fallback(MatchArgs a, cudaStream_t st) {
     return launch_global_m<M_SSD>(a, st);
 }
 
-cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st) {
+cudaError_t launch_match(MatchJob a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     const bool tiled = use_tiled && (a.bs == 4 || a.bs == 8);
     a.self_incl = a.radius == 0;
     const bool tc = metric == M_SSD && a.tc_ws != nullptr && tc_eligible(a);
     a.chunks = (2 * a.range + 1 + 3) / 4;
     a.tile_pitch = 128 + 4 * a.chunks;
-    if (a.zero[0] && (tc || !tiled || !scan_rows(a, metric, rows_per_cta))) {
+    if (a.zero.acc[0] && (tc || !tiled || !scan_rows(a, metric, rows_per_cta))) {
         for (int k = 0; k < 2; ++k)
-            if ((e = cudaMemsetAsync(a.zero[k], 0, (size_t)a.zero_count * 8, st)) != cudaSuccess) return e;
-        a.zero[0] = nullptr;
+            if ((e = cudaMemsetAsync(a.zero.acc[k], 0, (size_t)a.zero.count * 8, st)) != cudaSuccess) return e;
+        a.zero.acc[0] = nullptr;
     }
     if (tc) {
         // tensor-core bound + exact re-rank; the blocks it lists get the FP32 scan

@@ -227,21 +227,21 @@ inline size_t scan_tile_bytes(const MatchArgs &a, int rows_per_cta) {
            sizeof(float);
 }
 
-inline size_t scan_smem_bytes(const MatchArgs &a, int rows_per_cta) {
+inline size_t scan_smem_bytes(const MatchJob &a, int rows_per_cta) {
     return scan_tile_bytes(a, rows_per_cta) + (a.direct ? 0 : (size_t)kScanWarps * kPendBytes);
 }
 
 // CTA `part` of `parts` clears its share of the accumulators (16-byte stores; the arrays start
 // on 16 bytes).
-__device__ __forceinline__ void zero_slice(unsigned long long *const (&zero)[2], long long count, int part, int parts) {
-    if (!zero[0]) return;
-    const long long pairs = count / 2, per = (pairs + parts - 1) / parts;
+__device__ __forceinline__ void zero_slice(const ZeroArgs &zero, int part, int parts) {
+    if (!zero.acc[0]) return;
+    const long long pairs = zero.count / 2, per = (pairs + parts - 1) / parts;
     const long long first = per * part, last = min(first + per, pairs);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        ulonglong2 *z = reinterpret_cast<ulonglong2 *>(zero[k]);
+        ulonglong2 *z = reinterpret_cast<ulonglong2 *>(zero.acc[k]);
         for (long long i = first + threadIdx.x; i < last; i += blockDim.x) z[i] = make_ulonglong2(0, 0);
-        if (part == 0 && threadIdx.x == 0 && (count & 1)) zero[k][count - 1] = 0;
+        if (part == 0 && threadIdx.x == 0 && (zero.count & 1)) zero.acc[k][zero.count - 1] = 0;
     }
 }
 

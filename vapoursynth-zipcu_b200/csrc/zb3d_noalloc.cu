@@ -32,9 +32,9 @@ static __device__ __align__(256) unsigned char zb_noalloc_scratch[ZB_NOALLOC_BYT
 
 namespace zb {
 
-cudaError_t launch_match(MatchArgs a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st);
+cudaError_t launch_match(MatchJob a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st);
 size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
-int scan_shape(MatchArgs &a, int metric, bool full);
+int scan_shape(MatchJob &a, int metric, bool full);
 cudaError_t launch_filter(const FilterArgs &a, bool final_, int t2d, int t1d, cudaStream_t st);
 cudaError_t launch_finish(const unsigned long long *num, const unsigned long long *den, long long acc_plane_stride,
                           long long acc_frame_stride, int w, int h, int pitch, int nplanes, int tw,
@@ -137,7 +137,7 @@ extern "C" int zb3d_bm3d_plane_noalloc(const float *d_src, float *d_dst, int wid
     memcpy(&factor, &bits, 4);
     const float s = sigma * factor;
 
-    MatchArgs ma{};
+    MatchJob ma{};
     ma.frames = d_src;  // clip 0: the plane matched on (noisy, or the basic estimate)
     ma.fstride = (long long)pixels;
     ma.w = width;
@@ -150,13 +150,13 @@ extern "C" int zb3d_bm3d_plane_noalloc(const float *d_src, float *d_dst, int wid
     ma.nbx_al = (width - 8) / block_step + 1;
     ma.list = list;
     // the array keeps the previous call's sums: both accumulators start from zero
-    ma.zero[0] = num;
-    ma.zero[1] = den;
-    ma.zero_count = (long long)pixels;
+    ma.zero.acc[0] = num;
+    ma.zero.acc[1] = den;
+    ma.zero.count = (long long)pixels;
     bool tiled = block_step == 4 || block_step == 8;
     int rows = 4;
     if (tiled) {
-        MatchArgs t = ma;
+        MatchJob t = ma;
         t.chunks = (2 * bm_range + 1 + 3) / 4;
         t.tile_pitch = 128 + 4 * t.chunks;
         tiled = match_tile_bytes(t, 4) <= 200 * 1024;
