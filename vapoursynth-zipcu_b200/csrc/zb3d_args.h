@@ -82,7 +82,8 @@ struct BatchEntry {
     FilterArgs f;
     int tiles_x;                      // match items per tile row: m.tiles_x tiles, and one for the
                                       // clamped last block column where there is one
-    int match_items;                  // match tiles (kBatchMatchRows block rows each)
+    int rows, direct;                 // the match tiles' shape: block rows, and MatchJob::direct (8 rows)
+    int match_items;                  // match tiles
     int filter_items;                 // filter chunks (kBatchGroups groups each)
     long long first_match, first_filter;  // first item number of each kind
 };
@@ -105,7 +106,6 @@ struct BatchArgs {
 constexpr unsigned kSmemOptIn = 226 * 1024;
 
 constexpr int kBatchGroups = 32;      // groups per filter chunk
-constexpr int kBatchMatchRows = 8;    // block rows (warps) per match tile
 
 // Fixed-point scale of the accumulators: value * 2^32 held in a signed 64-bit sum.
 constexpr float kFixScale = 4294967296.0f;

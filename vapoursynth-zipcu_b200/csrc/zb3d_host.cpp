@@ -44,7 +44,8 @@ size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta);
 bool scan_rows_fit(const MatchJob &a, int metric, int rows_per_cta);
 bool scan_rows_fit2(const MatchJob &a, int metric, int rows_per_cta);
 int scan_shape(MatchJob &a, int metric, bool full);
-size_t batch_match_smem(const MatchJob &m);
+size_t scan_smem(const MatchJob &a, int rows);
+size_t scan_tile_smem(const MatchJob &a, int rows);
 cudaError_t launch_batch(const BatchArgs &b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st);
 cudaError_t filter_precision_init(int dev);
 size_t filter_precision_stack_floats(long long nblocks);
@@ -1012,26 +1013,24 @@ bool batch_eligible(const Filter *f, const Entry &en) {
         en.form != 0)
         return false;
     if (en.t2d != 0 || en.t1d != 0) return false;
-    MatchJob m{};
-    m.bs = en.bs;
-    m.range = en.range;
-    m.chunks = (2 * en.range + 1 + 3) / 4;
-    m.tile_pitch = 128 + 4 * m.chunks;
-    return scan_rows_fit(m, M_SSD, kBatchMatchRows);
+    return scan_tile_smem(scan_args(en, 0), 8) <= 200 * 1024;
 }
-
 
 struct BatchItem {
     int job;
     const Entry *en;
+    int rows = 0, direct = 0;  // work list: the match tiles' shape
 };
 
 // A batch's work list and scratch layout: eligible entries grouped by filter step (hard
-// threshold, Wiener), the others run on their own.
+// threshold, Wiener) and by whether two of their match CTAs share an SM (a launch has the shared
+// memory of its largest tile, so one wide search would halve the warps of all the others); the
+// other entries run on their own.
+constexpr int kBatchGroupKinds = 4;  // final, + 2: one CTA per SM
 struct BatchPlan {
     std::vector<zb3d_batch_job> jobs;
     int device = 0;
-    std::vector<BatchItem> groups[2], fallback;
+    std::vector<BatchItem> groups[kBatchGroupKinds], fallback;
     int nent = 0;
     size_t counters = 0, need = 0;
     std::vector<size_t> list_off, acc_off;
@@ -1064,21 +1063,26 @@ bool plan_batch(const zb3d_batch_job *jobs, int njobs, BatchPlan &p, char *err, 
     for (int j = 0; j < njobs; ++j) {
         const Filter *f = reinterpret_cast<const Filter *>(jobs[j].filter);
         for (const Entry &en : f->entries) {
-            if (batch_eligible(f, en)) p.groups[f->final_ ? 1 : 0].push_back({j, &en});
-            else p.fallback.push_back({j, &en});
+            MatchJob m = scan_args(en, 0);
+            const int rows = batch_eligible(f, en) ? scan_shape(m, M_SSD, true) : 0;
+            if (rows)
+                p.groups[(f->final_ ? 1 : 0) + (scan_rows_fit2(m, M_SSD, rows) ? 0 : 2)].push_back(
+                    {j, &en, rows, m.direct});
+            else
+                p.fallback.push_back({j, &en});
         }
     }
     // scratch layout: [counters | status | lists | accumulators]
-    p.nent = (int)(p.groups[0].size() + p.groups[1].size());
+    for (const auto &g : p.groups) p.nent += (int)g.size();
     p.counters = align256(4 * (size_t)std::max(p.nent, 1));
     p.need = p.counters + 256;
-    for (int g = 0; g < 2; ++g)
-        for (const BatchItem &it : p.groups[g]) {
+    for (const auto &g : p.groups)
+        for (const BatchItem &it : g) {
             p.list_off.push_back(p.need);
             p.need += align256((size_t)it.en->nblocks * 8 * sizeof(int2));
         }
-    for (int g = 0; g < 2; ++g)
-        for (const BatchItem &it : p.groups[g]) {
+    for (const auto &g : p.groups)
+        for (const BatchItem &it : g) {
             p.acc_off.push_back(p.need);
             p.need += 2 * align256((size_t)it.en->nplanes * it.en->plane_elems * 8);
         }
@@ -1181,7 +1185,7 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
     auto args = std::make_unique<BatchArgs>();
     int idx = 0;
     bool testing = unsatisfiable != 0;
-    for (int g = 0; g < 2; ++g)
+    for (int g = 0; g < kBatchGroupKinds; ++g)
         for (size_t at = 0; at < p.groups[g].size() && ce == cudaSuccess; at += kBatchEntries) {
             const int n = (int)std::min<size_t>(kBatchEntries, p.groups[g].size() - at), base = idx;
             size_t smem = 0;  // matching tiles
@@ -1236,11 +1240,13 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
                 const int nbw = en.bs == 4 ? 31 : 16;
                 m.tiles_x = (en.nbx_al + nbw - 1) / nbw;
                 B.tiles_x = m.tiles_x + (en.nbx_al != en.nbx ? 1 : 0);
-                B.match_items = B.tiles_x * ((en.nby + kBatchMatchRows - 1) / kBatchMatchRows);
+                B.rows = it.rows;
+                B.direct = it.direct;
+                B.match_items = B.tiles_x * ((en.nby + it.rows - 1) / it.rows);
                 B.filter_items = (int)((en.nblocks + kBatchGroups - 1) / kBatchGroups);
                 B.first_match = nm;
                 nm += B.match_items;
-                smem = std::max(smem, batch_match_smem(MatchJob{m}));
+                smem = std::max(smem, scan_smem(scan_args(en, it.direct), it.rows));
             }
             long long nf = nm;
             for (int i = 0; i < n; ++i) {
@@ -1255,7 +1261,7 @@ cudaError_t enqueue_batch(const BatchPlan &p, BatchBuffers &b, std::map<Filter *
             args->wait_polls = wait_polls ? wait_polls : (1u << 22);
             args->unsatisfiable = testing;
             testing = false;  // the first entry of the batch only
-            ce = launch_batch(*args, g == 1, 0, 0, smem, st);
+            ce = launch_batch(*args, (g & 1) != 0, 0, 0, smem, st);
             for (int i = 0; i < n && ce == cudaSuccess; ++i) {
                 const BatchItem &it = p.groups[g][at + i];
                 const Entry &en = *it.en;

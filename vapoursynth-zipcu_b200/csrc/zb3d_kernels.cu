@@ -442,12 +442,14 @@ __global__ void __launch_bounds__(PHASE == 1 ? kScanWarps * 32 : kFilter8Warps *
         const int bx = local % E.tiles_x, by = local / E.tiles_x;
         zero_slice(E.zero, local, E.match_items);
         if (bx == m.tiles_x) {  // the clamped last block column
-            const int cy = by * kBatchMatchRows + (threadIdx.x >> 5);
-            if (cy < m.nby) warp_block<M_SSD>(m, m.nbx - 1, cy);
-        } else if (m.bs == 4) {
-            scan_tile<M_SSD, true, 4, true>(m, bx, by, kBatchMatchRows, dyn);
+            const int warp = threadIdx.x >> 5, cy = by * E.rows + warp;
+            if (warp < E.rows && cy < m.nby) warp_block<M_SSD>(m, m.nbx - 1, cy);
+        } else if (E.direct) {
+            if (m.bs == 4) scan_tile<M_SSD, true, 4, false>(m, bx, by, kScanWarps, dyn);
+            else scan_tile<M_SSD, false, 8, false>(m, bx, by, kScanWarps, dyn);
         } else {
-            scan_tile<M_SSD, false, 8, true>(m, bx, by, kBatchMatchRows, dyn);
+            if (m.bs == 4) scan_tile<M_SSD, true, 4, true>(m, bx, by, E.rows, dyn);
+            else scan_tile<M_SSD, false, 8, true>(m, bx, by, E.rows, dyn);
         }
         __threadfence();  // each thread's list stores before the tile's count
         __syncthreads();
@@ -557,33 +559,21 @@ cudaError_t launch_finish(const unsigned long long *num, const unsigned long lon
     return cudaGetLastError();
 }
 
-// Bytes of dynamic shared memory a batch entry's matching needs (kBatchMatchRows block rows).
-size_t batch_match_smem(const MatchJob &m) { return scan_smem_bytes(m, kBatchMatchRows); }
-
-template <class K>
-static cudaError_t launch_batch_k(K k, const BatchArgs &b, long long items, int threads, size_t smem,
-                                  cudaStream_t st) {
-    if (items <= 0) return cudaSuccess;
-    // the same limit at every launch (see launch_scan_t), less the static buffers
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, k);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemOptIn - fa.sharedSizeBytes));
-    if (e != cudaSuccess) return e;
-    k<<<(unsigned)items, threads, smem, st>>>(b);
-    return cudaGetLastError();
-}
-
 // The batch kernels for the filter kind (final, t2d, t1d); only the DCT in both dimensions
 // is built in (other kinds run entry by entry).  match_smem: dynamic shared memory of the
 // match items.
 cudaError_t launch_batch(const BatchArgs &b, bool final_, int t2d, int t1d, size_t match_smem, cudaStream_t st) {
     if (t2d != T_DCT || t1d != T_DCT) return cudaErrorNotSupported;
-    cudaError_t e = launch_batch_k(final_ ? zb_batch<true, 1> : zb_batch<false, 1>, b, b.match_total, kScanWarps * 32,
-                                   match_smem, st);
+    if (b.match_total <= 0) return cudaSuccess;
+    auto match = zb_batch<false, 1>;  // the same for both filter kinds
+    // the same limit at every launch (see launch_scan_t)
+    cudaError_t e = cudaFuncSetAttribute(match, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemOptIn);
     if (e != cudaSuccess) return e;
-    return launch_batch_k(final_ ? zb_batch<true, 2> : zb_batch<false, 2>, b, b.items_total - b.match_total,
-                          kFilter8Warps * 32, 0, st);
+    match<<<(unsigned)b.match_total, kScanWarps * 32, match_smem, st>>>(b);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    auto filter = final_ ? zb_batch<true, 2> : zb_batch<false, 2>;
+    filter<<<(unsigned)(b.items_total - b.match_total), kFilter8Warps * 32, 0, st>>>(b);
+    return cudaGetLastError();
 }
 
 }  // namespace zb

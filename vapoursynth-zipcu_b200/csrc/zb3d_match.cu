@@ -348,6 +348,9 @@ bool scan_rows_fit2(const MatchJob &a, int metric, int rows_per_cta) {
     return scan_rows_fit(a, metric, rows_per_cta) && scan_smem_bytes(a, rows_per_cta) <= kSmemOptIn / 2;
 }
 
+size_t scan_smem(const MatchJob &a, int rows) { return scan_smem_bytes(a, rows); }
+size_t scan_tile_smem(const MatchJob &a, int rows) { return scan_tile_bytes(a, rows); }
+
 // The scan's shape without a timing: sets a.direct and returns the block rows per CTA (0: the
 // kernel takes no shape of the entry).  full: other planes fill the GPU beside this one.
 // 3840x2160 ssd, us (block_step 4 / 8; d8 and d4: inserted at once with 8 and 4 rows, q8 .. q1: queues):
