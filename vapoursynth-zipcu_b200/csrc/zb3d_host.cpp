@@ -410,17 +410,19 @@ bool alloc_slot(Filter *f, Slot &s) {
 }
 
 // Block matching of one entry into the slot's match list.
-// clear: the accumulators of the entry start from zero after it.
-cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, bool clear = false) {
+// clear: the accumulators of the entry start from zero after it.  spatial: the centre frame's
+// search alone (for timing).
+cudaError_t run_match(Filter *f, Slot &s, const Entry &en, const float *src, bool clear = false, bool spatial = false) {
         MatchJob ma{};
-        ma.frames = src;  // clip 0, plane 0: the matching plane of every window frame
+        // clip 0, plane 0: the matching plane of every window frame
+        ma.frames = src + (spatial ? (size_t)f->radius * en.plane_elems : 0);
         ma.fstride = (long long)en.plane_elems;
         ma.w = en.w;
         ma.h = en.h;
         ma.pitch = en.pitch;
         ma.bs = en.bs;
         ma.range = en.range;
-        ma.radius = f->radius;
+        ma.radius = spatial ? 0 : f->radius;
         ma.ps_num = en.ps_num;
         ma.ps_range = en.ps_range;
         ma.nbx = en.nbx;
@@ -542,8 +544,9 @@ long long scan_ctas(const Entry &e, int rows) {
 // whatever the rows; fewer rows split each block's candidate rows, which helps a plane whose
 // CTAs do not fill the GPU) or with candidates inserted at once (a warp per row, and less shared
 // memory: better where the queues would leave one CTA per SM, and at small ranges, where the
-// tile's load counts most); or the tensor-core form (ssd, where eligible); by timing each on a
-// synthetic plane of the entry's geometry with slot s's buffers.
+// tile's load counts most); or the tensor-core form (ssd, where eligible); by timing the spatial
+// search of each, which is all that they differ in, on a synthetic plane of the entry's geometry
+// with slot s's buffers.
 void tune_entry(Filter *f, Slot &s, Entry &e) {
     e.rows = 4;
     MatchArgs ga{};
@@ -630,7 +633,7 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     for (int t = 0; ok && t < f->tw; ++t)
         ok = cudaMemcpy(s.d_src + e.src_off + (size_t)t * e.plane_elems, host.data(), host.size() * sizeof(float),
                         cudaMemcpyHostToDevice) == cudaSuccess;
-    float best_ms = 3.0e38f;  // of the shapes with queues, and the tensor-core form
+    float best_ms = 3.0e38f;  // of the FP32 shapes that are not inserted at once
     Shape best{-1, e.rows, 0};
     std::vector<std::pair<float, Shape>> times;
     for (const auto &cand : cands) {
@@ -643,7 +646,7 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
         bool good = true;
         for (int it2 = 0; it2 < 4 && good; ++it2) {
             good = cudaEventRecord(a, s.st) == cudaSuccess &&
-                   run_match(f, s, t, s.d_src + e.src_off, true) == cudaSuccess &&  // with the accumulators' zeros
+                   run_match(f, s, t, s.d_src + e.src_off, true, true) == cudaSuccess &&  // with the accumulators' zeros
                    cudaEventRecord(b, s.st) == cudaSuccess &&
                    cudaEventSynchronize(b) == cudaSuccess;
             float ms = 0.0f;
@@ -653,10 +656,10 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
             cudaGetLastError();
             continue;
         }
-        if (!cand.direct && lo < best_ms) best_ms = lo;
+        if (cand.form == 0 && !cand.direct && lo < best_ms) best_ms = lo;
         times.push_back({lo, cand});
     }
-    // The first candidate within 20% of the fastest: fewer block rows per CTA make one plane's
+    // Of the shapes with queues the first within 20% of the fastest: fewer block rows per CTA make one plane's
     // launch shorter by filling the GPU, but cost more in all (every range of candidate rows
     // builds a list of its own), which shows as soon as other streams fill it (640x480 at
     // block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3 streams).
@@ -664,19 +667,21 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     const float slack = entry_scan_fits(e, 1) && scan_ctas(e, 1) > sms ? 1.2f : 1.0f;
     float chosen_ms = 3.0e38f;
     for (const auto &t : times)
-        if (best.form < 0 && !t.second.direct && t.first <= slack * best_ms) {
+        if (best.form < 0 && t.second.form == 0 && !t.second.direct && t.first <= slack * best_ms) {
             best = t.second;
             chosen_ms = t.first;
         }
     // Inserted at once: where it is clearly faster alone.  With other streams beside it a few
     // per cent do not last (1080p block_step 4, bm_range 12, 4% alone: two passes 1301 us with
     // queues, 1312 without; block_step 8, bm_range 9, 13% alone: Wiener 256 and 247 us).
-    chosen_ms *= 0.93f;
+    const float clear_ms = 0.93f * chosen_ms;
     for (const auto &t : times)
-        if (t.second.direct && t.first < chosen_ms) {
+        if (t.second.direct && t.first < std::min(chosen_ms, clear_ms)) {
             best = t.second;
             chosen_ms = t.first;
         }
+    for (const auto &t : times)  // the tensor-core form: where it is faster
+        if (t.second.form == 1 && t.first < chosen_ms) best = t.second;
     ok = ok && best.form >= 0;
     if (a) cudaEventDestroy(a);
     if (b) cudaEventDestroy(b);
