@@ -11,7 +11,9 @@ enum Metric { M_SSD = 0, M_SAD = 1, M_ZSSD = 2, M_ZSAD = 3, M_SSD_NORM = 4 };
 // A kernel argument of at most 128 bytes: with a larger one nvcc compiles every kernel that takes
 // it to other registers (sad scan from global memory 126 -> 120, general temporal search of ssd
 // with 8 entries 228 -> 464 bytes of spills), and those were up to 18% slower.  What only the
-// launchers or one kernel want is in MatchJob.
+// launchers or one kernel want is in MatchJob.  Two kernels are better with the larger argument
+// and take a MatchJob: the temporal rows kernel (1920x1080, radius 2: 2 us) and the tensor-core
+// form (no spills; 32 bytes with MatchArgs).
 struct MatchArgs {
     const float *frames;   // matching plane of window frame t at frames + t*fstride
     long long fstride;
@@ -50,7 +52,7 @@ struct ZeroArgs {
     long long count;
 };
 
-// What launch_match takes.
+// What launch_match takes, and the argument of zb_match_temporal_rows and zb_match_tc.
 struct MatchJob : MatchArgs {
     ZeroArgs zero;
     int direct;            // scan kernel: 1 = a warp per block row, candidates inserted at once; 0 = 8 warps, queues

@@ -36,7 +36,7 @@ namespace zb {
 
 cudaError_t launch_match(MatchJob a, int metric, int rows_per_cta, bool use_tiled, cudaStream_t st);
 bool tc_eligible(const MatchArgs &a);
-cudaError_t launch_match_tc(const MatchArgs &a, cudaStream_t st);
+cudaError_t launch_match_tc(const MatchJob &a, cudaStream_t st);
 cudaError_t launch_tc_fallback(MatchArgs a, cudaStream_t st);
 int tc_debug_cols(const MatchArgs &a);
 int pilot_device(const zb3d_pilot *p);
@@ -1981,8 +1981,8 @@ int zb3d_match_stats(zb3d_filter *fp, unsigned long long out[4], int reset) {
     return 0;
 }
 
-static zb::MatchArgs probe_args(int width, int height, int pitch, int bs, int range) {
-    zb::MatchArgs a{};
+static zb::MatchJob probe_args(int width, int height, int pitch, int bs, int range) {
+    zb::MatchJob a{};
     a.w = width;
     a.h = height;
     a.pitch = pitch;
@@ -2010,7 +2010,7 @@ int zb3d_tc_probe(const float *d_plane, int width, int height, int pitch, int bl
         set_err(err, errlen, "zb3d_tc_probe: bad geometry.");
         return -1;
     }
-    MatchArgs a = probe_args(width, height, pitch, block_step, bm_range);
+    MatchJob a = probe_args(width, height, pitch, block_step, bm_range);
     if (!tc_eligible(a)) return 1;
     a.frames = d_plane;
     a.list = reinterpret_cast<int2 *>(d_list);

@@ -461,9 +461,9 @@ size_t match_tile_bytes(const MatchArgs &a, int rows_per_cta) {
 }
 
 bool tc_eligible(const MatchArgs &a);                          // zb3d_match_tc.cu
-cudaError_t launch_match_tc(const MatchArgs &a, cudaStream_t st);
+cudaError_t launch_match_tc(const MatchJob &a, cudaStream_t st);
 bool temporal_rows_eligible(const MatchArgs &a, int metric);   // zb3d_match_temporal.cu
-cudaError_t launch_temporal_rows(const MatchArgs &a, cudaStream_t st);
+cudaError_t launch_temporal_rows(const MatchJob &a, cudaStream_t st);
 
 // The FP32 scan of the blocks the tensor-core kernel listed (SSD, radius 0).
 cudaError_t launch_tc_fallback(MatchArgs a, cudaStream_t st) {

@@ -352,7 +352,7 @@ __device__ __forceinline__ void stage_region(float *reg, int cap, const float *p
 // of warp MMA_WARP issues the MMAs.  The roles meet at mbarriers: done[s] (MMAs of the
 // job complete, tcgen05.commit) and free[s] (the slot read by the block warps of its
 // parity); job j waits for phase (j / 2) mod 2.
-__global__ void __launch_bounds__(THREADS, 1) zb_match_tc(MatchArgs a) {
+__global__ void __launch_bounds__(THREADS, 1) zb_match_tc(MatchJob a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const Geom g = tile_geom(a);
@@ -932,7 +932,7 @@ bool tc_eligible(const MatchArgs &a) {
            15 * a.bs + 2 * a.range + 1 <= tc::MAX_UR;
 }
 
-cudaError_t launch_match_tc(const MatchArgs &a, cudaStream_t st) {
+cudaError_t launch_match_tc(const MatchJob &a, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(a.tc_ws, 0, kTcWsList * sizeof(int), st);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(tc::zb_match_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);

@@ -156,7 +156,7 @@ __device__ __forceinline__ void scan_window_group(const MatchArgs &a, int xx, in
 }
 
 template <int P>
-__global__ void __launch_bounds__(kTempWarps * 32, 4) zb_match_temporal_rows(MatchArgs a) {
+__global__ void __launch_bounds__(kTempWarps * 32, 4) zb_match_temporal_rows(MatchJob a) {
     using S = TempShape<P>;
     constexpr int G = S::G, NG = S::NG;
     __shared__ float wins[kTempWarps * 2 * S::BUF];
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kTempWarps * 32, 4) zb_match_temporal_rows(Mat
 }
 
 template <int P>
-static cudaError_t launch_rows_t(const MatchArgs &a, cudaStream_t st) {
+static cudaError_t launch_rows_t(const MatchJob &a, cudaStream_t st) {
     const long long nb = (long long)a.nby * a.nbx;
     const int per = kTempWarps * TempShape<P>::NG;
     zb_match_temporal_rows<P><<<(unsigned)((nb + per - 1) / per), kTempWarps * 32,
@@ -286,7 +286,7 @@ bool temporal_rows_eligible(const MatchArgs &a, int metric) {
     return metric == M_SSD && a.ps_num >= 1 && a.ps_num <= 2 && a.ps_range >= 2 && a.ps_range <= 6;
 }
 
-cudaError_t launch_temporal_rows(const MatchArgs &a, cudaStream_t st) {
+cudaError_t launch_temporal_rows(const MatchJob &a, cudaStream_t st) {
     switch (a.ps_range) {
     case 2: return launch_rows_t<2>(a, st);
     case 3: return launch_rows_t<3>(a, st);
