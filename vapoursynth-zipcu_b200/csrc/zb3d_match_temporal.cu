@@ -281,9 +281,13 @@ static cudaError_t launch_rows_t(const MatchJob &a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Whether the row kernel takes this search: window rows that fill a warp well.
+// Whether the row kernel takes this search: window rows that fill a warp well, in a plane of more
+// than 4 candidate positions (it scans whole windows: 8x8, 1 position, radius 3, ps_range 4: 37 us a
+// search, 14.5 with a lane pair per block, which scans the positions that exist; 10x10, 9
+// positions: equal).
 bool temporal_rows_eligible(const MatchArgs &a, int metric) {
-    return metric == M_SSD && a.ps_num >= 1 && a.ps_num <= 2 && a.ps_range >= 2 && a.ps_range <= 6;
+    return metric == M_SSD && a.ps_num >= 1 && a.ps_num <= 2 && a.ps_range >= 2 && a.ps_range <= 6 &&
+           (long long)(a.w - 7) * (a.h - 7) > 4;
 }
 
 cudaError_t launch_temporal_rows(const MatchJob &a, cudaStream_t st) {
