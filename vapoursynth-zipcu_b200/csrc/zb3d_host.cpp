@@ -585,7 +585,7 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     // 1080p radius 2 window) such a CTA writes before it starts, with no other CTA's arithmetic
     // to hide them (three windows in flight: 381 us a window with queues, 391 without)
     if (!cands.empty() && f->radius == 0)
-        for (int r = 8; r >= 2; r >>= 1)
+        for (int r : {8, 4})  // 2 rows were never the faster
             if (entry_scan_fits(e, r, 1)) cands.push_back({0, r, 1});
     if (tc_ok && f->match_form != 0) cands.push_back({1, 4, 0});
     if (cands.size() < 2) return;
