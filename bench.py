@@ -975,7 +975,7 @@ def run_batched(torch, steps: int, warmup: int, nstreams: int = 4):
         lat[ci].append(a.elapsed_time(z))
     px = sum(c["w"] * c["h"] * nfr for c in clips) * steps
     # the same step through zb3d_process_batch: one call per 16 windows (a frame of every clip
-    # x 4 frames), each a persistent work-list launch over the windows' eligible planes (the
+    # x 4 frames), each two work-list launches over the windows' eligible planes (the
     # r1 clip's planes run entry by entry inside the call); latency per call
     from zb3d.device import process_batch
     bst = torch.cuda.Stream()
@@ -1189,11 +1189,12 @@ def main():
     props = torch.cuda.get_device_properties(local)
     peak_fp32 = props.multi_processor_count * 128 * 2 * sm_max * 1e6 / 1e12
     achieved = match_flops_total / (match_ms / 1e3) / 1e12 if match_ms > 0 else None
-    # DRAM bytes per matching launch: ncu measured 8.32 MB read and 0 written for the
-    # 1920x1080 Y launch, which is the plane read once (4 B per pixel); scaled by plane
-    # size to the average of the batch's Y, U and V launches
+    # DRAM bytes per matching launch: ncu measured 8.37 MB read and up to 0.49 MB written for the
+    # 1920x1080 Y launch: the plane read once (4 B per pixel), and the accumulators' 33 MB of
+    # zeros, which it stores too, nearly all still in L2 when it ends; scaled by plane size to
+    # the average of the batch's Y, U and V launches
     plane_px = [w * h for (w, h) in plane_dims()]
-    traffic = 8.32e6 * (sum(plane_px) / len(plane_px)) / plane_px[0]
+    traffic = 8.86e6 * (sum(plane_px) / len(plane_px)) / plane_px[0]
 
     out = {"metric": METRIC, "value": value, "unit": "Mpix/s", "n_gpus": world, "steps": args.steps,
            "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -1210,9 +1211,10 @@ def main():
            "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak_fp32, "unit": "TFLOP/s",
                         "frac": (achieved / peak_fp32) if achieved else None, "traffic": traffic,
                         "traffic_how": "DRAM read + write bytes per launch from an ncu capture of the 1920x1080 Y "
-                                       "launch (8.32 MB read, 0 written), scaled by plane size to the average "
-                                       "launch; algorithmically the plane is read once",
-                        "kernel": "zb_match_tiled2<shared, bs4> (block matching, packed FP32x2)",
+                                       "launch (8.37 MB read, up to 0.49 MB written), scaled by plane size to the "
+                                       "average launch; algorithmically the plane is read once; the launch also "
+                                       "stores 33 MB of accumulator zeros, which stay in L2",
+                        "kernel": "zb_match_scan<ssd, shared, bs4> (block matching, packed FP32x2)",
                         "per_launch_ms": match_ms / max(match_n, 1), "launches": match_n,
                         "how": "algorithmic FLOP (192 per candidate, all clipped windows) of one batch's "
                                "matching launches / their CUDA-event time, one stream, after the timed region",
