@@ -1082,7 +1082,7 @@ def run_batched(torch, steps: int, warmup: int, nstreams: int = 4):
             "config": {"workload": "4 clips x 16 frames: 720x480 YUV420 r0, 1280x720 YUV444 CBM3D r0, 1280x720 "
                                    "YUV420 r1 (stacked output), 3840x2160 YUV420 r0; sigma U[5,20] per clip; "
                                    "block_step 4, bm_range 12, single pass", "streams": nstreams,
-                       "launch": "one CUDA graph per window (all planes' memsets, matching, filtering, finishing)",
+                       "launch": "one CUDA graph per window (all planes' matching, filtering, finishing)",
                        "per_clip": per_clip},
             "batch_form": batch_form}
 

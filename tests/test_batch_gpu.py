@@ -1,4 +1,5 @@
-"""zb3d_process_batch: one persistent launch over the plane entries of many windows.
+"""zb3d_process_batch: two work-list launches (matching, filtering) per filter kind over the plane
+entries of many windows.
 
 * The outputs of a batch of uneven jobs equal, byte for byte, each job run on its own
   through zb3d_process_device. The jobs cover luma and chroma planes of different sizes,

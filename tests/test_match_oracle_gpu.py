@@ -3,10 +3,10 @@ test_ref_pin.py pins to the reference kernels), on paths the parity configuratio
 reach:
 
 * the packed tile's half-plane layout sized at run time (bm_range > 15 at block_step 4 and
-  8), with ragged widths (the clamped last block column) and both the default CTA shape and
-  the one the autotuner picks (2, 4 or 8 block rows);
-* the temporal search with per-frame lists of 2 entries (ps_num 1 and 2) and of 8 entries
-  (ps_num 3 and 5), over moving frames.
+  8), with ragged widths (the clamped last block column) and both the untimed CTA shape and
+  the one the autotuner picks;
+* the temporal search by rows (ps_num 1 and 2) and by lane pairs with per-frame lists of 8
+  entries (ps_num 3 and 5), over moving frames.
 """
 import numpy as np
 import pytest

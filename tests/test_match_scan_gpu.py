@@ -79,7 +79,7 @@ def test_scan_lists_equal_oracle(w, h, bs, R, metric, kind, rows, monkeypatch, t
 
 
 def test_threads_with_differently_shaped_launches(monkeypatch, tmp_path):
-    """Planes of one clip with 8, 4 and 2 block rows per CTA (other shared-memory sizes of the same
+    """Planes of one clip with 8 and 2 block rows per CTA (other shared-memory sizes of the same
     kernel), requested by 8 threads over 4 streams: every frame comes, and is the frame of one thread."""
     w, h, nf = 256, 144, 24
     add = force_rows(monkeypatch, tmp_path / "tune.txt", 8)

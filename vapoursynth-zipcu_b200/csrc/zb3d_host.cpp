@@ -710,8 +710,8 @@ cudaError_t run_entry(Filter *f, Slot &s, const Entry &en, const float *src, flo
 cudaError_t run_entry_steps(Filter *f, Slot &s, const Entry &en, const float *src, float *dst);
 
 // Runs `fn(s)` (launches on s.st) as a CUDA graph: captured once per key on the slot's
-// own stream, then replayed on `launch`.  A window's whole launch sequence (memsets,
-// matching, filtering, finishing of every plane) becomes one graph launch.  Graphs bake
+// own stream, then replayed on `launch`.  A window's whole launch sequence
+// (matching, filtering, finishing of every plane) becomes one graph launch.  Graphs bake
 // in the slot's scratch buffers, so replays of one key must not overlap (the device
 // entry points' rule).  ZB3D_GRAPHS=0, profiling, or a failed capture -> direct launches.
 template <class Fn>
@@ -978,8 +978,8 @@ using zb::Filter;
 namespace zb {
 namespace {
 
-// Scratch of a batch: per-entry match lists and accumulators, the entry table, item
-// counters and the status word.  The synchronous call shares one per device (grown on
+// Scratch of a batch: per-entry match lists and accumulators, the counters of finished match
+// tiles and the status word.  The synchronous call shares one per device (grown on
 // demand); a graph handle owns its own.
 struct BatchBuffers {
     char *arena = nullptr;

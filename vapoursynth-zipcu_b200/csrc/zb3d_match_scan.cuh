@@ -25,10 +25,12 @@
 // multiply-adds of two cycles each, and the joins); with queues 73% of active cycles at 1920x1080,
 // block_step 4, bm_range 12, whose 544 CTAs are 1.84 waves.  The queues' 32 KB decide how many
 // CTAs share an SM, so where that costs more than they save candidates are inserted at once:
-// 1080p us at block_step 4 / 8, inserted at once and queued (8 rows, ssd): bm_range 9 174 / 97 and
-// 185 / 119, bm_range 12 275 / 149 and 284 / 175, bm_range 24 1184 / 601 and 1049 / 544.  Small
-// planes take queues for their ranges of candidate rows: 320x240 at block_step 4, bm_range 12: 92
-// at once, 40 with 8 ranges.  scan_shape (zb3d_match.cu) has the rule, and the autotuner times both.
+// 1080p us at block_step 4 / 8, inserted at once and queued (8 rows, ssd, a noisy plane of
+// gradients): bm_range 9 174 / 97 and 185 / 119, bm_range 12 275 / 149 and 284 / 175, bm_range 24
+// 1184 / 601 and 1049 / 544; 326 before the column stream (block_step 4, bm_range 12, textured
+// plane; 291 now, queued).  Small planes take queues for their ranges of candidate rows: 320x240
+// at block_step 4, bm_range 12: 92 at once, 40 with 8 ranges.  scan_shape (zb3d_match.cu) has the
+// rule, and the autotuner times both.
 #pragma once
 #include "zb3d_match.cuh"
 
