@@ -413,29 +413,7 @@ __device__ __forceinline__ void warp_block(const MatchArgs &a, int kx, int by) {
         }
     }
     if (lane != 0) return;
-    const long long bi = (long long)by * a.nbx + kx;
-    const int self = pack_pos(x, y);
-    if (a.self_incl) {
-        bool found = false;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) found |= (q[i] == self);
-        if (!found) {
-#pragma unroll
-            for (int i = 7; i > 0; --i) {
-                e[i] = e[i - 1];
-                q[i] = q[i - 1];
-            }
-            e[0] = 0.0f;
-            q[0] = self;
-        }
-    }
-    const int zr = a.radius << 24;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) a.list[bi * 8 + i] = make_int2(pos_x(q[i]), pos_y(q[i]) | zr);
-    if (a.errs) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a.errs[bi * 8 + i] = e[i];
-    }
+    store_list(a, (long long)by * a.nbx + kx, x, y, e, q);
 }
 
 }  // namespace zb
