@@ -633,8 +633,6 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
     for (int t = 0; ok && t < f->tw; ++t)
         ok = cudaMemcpy(s.d_src + e.src_off + (size_t)t * e.plane_elems, host.data(), host.size() * sizeof(float),
                         cudaMemcpyHostToDevice) == cudaSuccess;
-    // with the accumulators' zeros where a shape decides how they are written
-    const bool scan = entry_scan_fits(e, 1);
     float best_ms = 3.0e38f;  // of the FP32 shapes that are not inserted at once
     Shape best{-1, e.rows, 0};
     std::vector<std::pair<float, Shape>> times;
@@ -648,9 +646,8 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
         bool good = true;
         for (int it2 = 0; it2 < 4 && good; ++it2) {
             good = cudaEventRecord(a, s.st) == cudaSuccess &&
-                   run_match(f, s, t, s.d_src + e.src_off, scan, true) == cudaSuccess &&
-                   cudaEventRecord(b, s.st) == cudaSuccess &&
-                   cudaEventSynchronize(b) == cudaSuccess;
+                   run_match(f, s, t, s.d_src + e.src_off, false, true) == cudaSuccess &&
+                   cudaEventRecord(b, s.st) == cudaSuccess && cudaEventSynchronize(b) == cudaSuccess;
             float ms = 0.0f;
             if (good && cudaEventElapsedTime(&ms, a, b) == cudaSuccess && it2 > 0) lo = std::min(lo, ms);
         }
@@ -661,12 +658,12 @@ void tune_entry(Filter *f, Slot &s, Entry &e) {
         if (cand.form == 0 && !cand.direct && lo < best_ms) best_ms = lo;
         times.push_back({lo, cand});
     }
-    // Of the shapes with queues the first within 20% of the fastest: fewer block rows per CTA make one plane's
-    // launch shorter by filling the GPU, but cost more in all (every range of candidate rows
-    // builds a list of its own), which shows as soon as other streams fill it (640x480 at
-    // block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3 streams).
-    // A plane that leaves SMs without a CTA even at one row takes the fastest.
-    const float slack = scan && scan_ctas(e, 1) > sms ? 1.2f : 1.0f;
+    // Of the shapes with queues the first within 20% of the fastest: fewer block rows per CTA make
+    // one plane's launch shorter by filling the GPU, but cost more in all (every range of
+    // candidate rows builds a list of its own), which shows as soon as other streams fill it
+    // (640x480 at block_step 8: 2 rows 39 us, 1 row 34 us alone; 28.1 and 31.5 us a window on 3
+    // streams).  A plane that leaves SMs without a CTA even at one row takes the fastest.
+    const float slack = entry_scan_fits(e, 1) && scan_ctas(e, 1) > sms ? 1.2f : 1.0f;
     float chosen_ms = 3.0e38f;
     for (const auto &t : times)
         if (best.form < 0 && t.second.form == 0 && !t.second.direct && t.first <= slack * best_ms) {
